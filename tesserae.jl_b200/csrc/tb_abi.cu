@@ -482,7 +482,7 @@ int run_step(tb_ctx* c, const tb_mesh* m, tb_particles* p, tb_partition* part, t
              const tb_step_params* prm, int nsteps, bool do_bin, bool do_p2g, bool do_grid, bool do_g2p,
              bool x64 = false, double reorder_threshold = 0.0) {
     auto M = make_dmesh<D, T>(*m);
-    auto S = make_scalars<T>(*prm);
+    auto S = make_scalars<T>(*prm, *m);
     PView<T> P;
     GView<T> G;
     int rc;
@@ -684,7 +684,7 @@ int do_weights(tb_ctx* c, const tb_mesh* m, const tb_particles* p, const tb_step
     if (!w || (p && p->n && (!w->w || !w->grad_w || !w->window))) return fail(c, TB_ERR_ARG, "weights array is NULL");
     PView<T> P;
     if ((rc = make_pview<T>(c, p, m->dim, false, false, P)) != TB_OK) return rc;
-    auto S = make_scalars<T>(*prm);
+    auto S = make_scalars<T>(*prm, *m);
     const LaunchCfg cfg = cfg_of(c);
     cudaError_t e;
     if (m->dim == 3)
@@ -708,11 +708,11 @@ int do_grid_update(tb_ctx* c, const tb_mesh* m, tb_grid* g, const tb_step_params
     if ((rc = make_gview<T>(c, g, m->dim, G, m->block_log2)) != TB_OK) return rc;
     c->grid_sparse_ok = false;  // a standalone call cannot know which nodes are non-zero
     if (m->dim == 3)
-        e = grid_update_sparse_or_dense<3, T, 4>(c, make_dmesh<3, T>(*m), G, make_scalars<T>(*prm), cfg);
+        e = grid_update_sparse_or_dense<3, T, 4>(c, make_dmesh<3, T>(*m), G, make_scalars<T>(*prm, *m), cfg);
     else if (m->block_log2 == 3)
-        e = grid_update_sparse_or_dense<2, T, 8>(c, make_dmesh<2, T>(*m), G, make_scalars<T>(*prm), cfg);
+        e = grid_update_sparse_or_dense<2, T, 8>(c, make_dmesh<2, T>(*m), G, make_scalars<T>(*prm, *m), cfg);
     else
-        e = grid_update_sparse_or_dense<2, T, 4>(c, make_dmesh<2, T>(*m), G, make_scalars<T>(*prm), cfg);
+        e = grid_update_sparse_or_dense<2, T, 4>(c, make_dmesh<2, T>(*m), G, make_scalars<T>(*prm, *m), cfg);
     return e == cudaSuccess ? TB_OK : cuda_fail(c, e, "grid update launch");
 }
 
@@ -728,8 +728,8 @@ int do_g2p_direct(tb_ctx* c, const tb_mesh* m, const tb_grid* g, tb_particles* p
         return rc;
     if ((rc = make_gview<T>(c, g, m->dim, G, m->block_log2)) != TB_OK) return rc;
     const LaunchCfg cfg = cfg_of(c);
-    cudaError_t e = (m->dim == 3) ? launch_g2p_direct<3, T>(make_dmesh<3, T>(*m), G, P, make_scalars<T>(*prm), cfg)
-                                  : launch_g2p_direct<2, T>(make_dmesh<2, T>(*m), G, P, make_scalars<T>(*prm), cfg);
+    cudaError_t e = (m->dim == 3) ? launch_g2p_direct<3, T>(make_dmesh<3, T>(*m), G, P, make_scalars<T>(*prm, *m), cfg)
+                                  : launch_g2p_direct<2, T>(make_dmesh<2, T>(*m), G, P, make_scalars<T>(*prm, *m), cfg);
     return e == cudaSuccess ? TB_OK : cuda_fail(c, e, "g2p launch");
 }
 
@@ -886,7 +886,9 @@ int do_wave_speed(tb_ctx* c, int32_t dim, const tb_particles* p, const tb_step_p
     cudaError_t e = cudaSuccess;
     if (!c->wave_max) e = cudaMalloc(&c->wave_max, sizeof(unsigned long long));
     if (e != cudaSuccess) return cuda_fail(c, e, "cudaMalloc wave speed");
-    const auto S = make_scalars<T>(*prm);
+    tb_mesh unit{};  // the wave speed reads no length
+    unit.h = 1.0;
+    const auto S = make_scalars<T>(*prm, unit);
     e = dim == 3 ? launch_wave_speed<3, T>(P, S, c->wave_max, cfg_of(c)) : launch_wave_speed<2, T>(P, S, c->wave_max, cfg_of(c));
     unsigned long long bits = 0;
     if (e == cudaSuccess) e = cudaMemcpyAsync(&bits, c->wave_max, sizeof bits, cudaMemcpyDeviceToHost, c->stream);
@@ -907,7 +909,7 @@ template <int D, class T, int BW>
 int g2p2g_impl(tb_ctx* c, const tb_mesh* m, tb_particles* p, tb_partition* part, tb_grid* g,
                const tb_step_params* prm, bool x64) {
     const auto M = make_dmesh<D, T>(*m);
-    const auto S = make_scalars<T>(*prm);
+    const auto S = make_scalars<T>(*prm, *m);
     PView<T> P;
     GView<T> G;
     int rc;
@@ -1037,7 +1039,7 @@ int adjoint_impl(tb_ctx* c, const tb_mesh* m, tb_particles* p, tb_partition* par
         totals = c->d_totals;
     }
     const auto M = make_dmesh<D, T>(*m);
-    const auto S = make_scalars<T>(*prm);
+    const auto S = make_scalars<T>(*prm, *m);
     PView<T> P;
     GView<T> G;
     AdjView A;

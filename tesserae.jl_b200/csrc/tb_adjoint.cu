@@ -63,11 +63,15 @@ template <int D, class T>
 __device__ __forceinline__ bool adj_axes(const DMesh<D, T>& M, const Scalars<T>& s, const double* xd, bool x64,
                                          T l_abs, AdjAxes<D>& A, int* err) {
     Basis<D, T> B;
+    GimpLen<T> gl;
+    gl.ln = l_abs / M.h;
+    gl.il = T(1) / gl.ln;
+    gl.ln64 = double(l_abs) / M.h64;
     if (x64) {
-        if (!prepare_basis_x64<D, T>(M, s.basis, xd, l_abs, B, err)) return false;
+        if (!prepare_basis_x64<D, T>(M, s.basis, xd, gl, B, err)) return false;
     } else {
         const T x[3] = {T(xd[0]), T(xd[1]), T(xd[2])};
-        if (!prepare_basis<D, T, false>(M, s.basis, x, l_abs, B, err)) return false;
+        if (!prepare_basis<D, T, false>(M, s.basis, x, gl, B, err)) return false;
     }
     const bool gimp = s.basis == TB_UGIMP;
     const double lnorm = gimp ? (x64 ? double(l_abs) / M.h64 : double(T(l_abs / M.h))) : 0.0;
@@ -485,12 +489,12 @@ __global__ void __launch_bounds__(SC_THREADS, 1) adj_scatter_kernel(DMesh<D, T> 
             pid[u] = (tid + u * NT < SC_NR && q < c1) ? perm[q] - 1 : -1;
         }
         double px[ITEMS][3];
-        T pl[ITEMS];
+        GimpLen<T> pl[ITEMS];
 #pragma unroll
         for (int u = 0; u < ITEMS; ++u) {
             const long long p = pid[u] >= 0 ? pid[u] : 0;
             load_xd<D, T>(P, p, px[u]);
-            pl[u] = (pid[u] >= 0 && P.l) ? P.l[p] : s.gimp_l;
+            pl[u] = pid[u] >= 0 ? gimp_len(M, P, s, p) : s.gimp;
         }
         // the coefficients go to the record slot at once (used only if the
         // window lands in the tile)
@@ -930,14 +934,18 @@ __device__ __forceinline__ bool dual_basis(const DMesh<D, Dual3>& MD, const Scal
         xd[d] = Dual3(d < D ? x[d] : 0.0);
         if (d < D) xd[d].d[d] = 1.0;
     }
-    return prepare_basis<D, Dual3, true>(MD, s.basis, xd, Dual3(double(l)), B, err);
+    GimpLen<Dual3> gl;
+    gl.ln64 = double(l) / MD.h.v;
+    gl.ln = Dual3(gl.ln64);
+    gl.il = Dual3(1.0 / gl.ln64);
+    return prepare_basis<D, Dual3, true>(MD, s.basis, xd, gl, B, err);
 }
 
-// N, grad N (values and x_p derivatives) at window slot (i, j, k), r = X - x_p.
+// N, grad N (values and x_p derivatives) at window slot (i, j, k).
 template <int D>
 __device__ __forceinline__ void dual_node(const DMesh<D, Dual3>& MD, const Basis<D, Dual3>& B, int i, int j, int k,
-                                          const Dual3* rel, Dual3& N, Dual3* G) {
-    eval_node<D, Dual3>(MD, B, i, j, k, rel, N, G);
+                                          Dual3& N, Dual3* G) {
+    eval_node<D, Dual3>(MD, B, i, j, k, N, G);
 }
 
 template <int D, class T>
@@ -987,7 +995,7 @@ __global__ void __launch_bounds__(128) adj_g2p_gen_kernel(DMesh<D, T> M, GView<T
                         node_of(i, j, k, I, rel, valid);
                         if (!valid) continue;
                         Dual3 N, Gn[3];
-                        dual_node<D>(MD, B, i, j, k, rel, N, Gn);
+                        dual_node<D>(MD, B, i, j, k, N, Gn);
 #pragma unroll
                         for (int r = 0; r < D; ++r)
 #pragma unroll
@@ -1036,7 +1044,7 @@ __global__ void __launch_bounds__(128) adj_g2p_gen_kernel(DMesh<D, T> M, GView<T
                         node_of(i, j, k, I, rel, valid);
                         if (!valid) continue;
                         Dual3 N, Gn[3];
-                        dual_node<D>(MD, B, i, j, k, rel, N, Gn);
+                        dual_node<D>(MD, B, i, j, k, N, Gn);
                         double vi[3] = {}, vni[3] = {};
 #pragma unroll
                         for (int d = 0; d < D; ++d) {
@@ -1139,7 +1147,7 @@ __global__ void __launch_bounds__(128) adj_p2g_gen_kernel(DMesh<D, T> M, PView<T
                         rel[d].d[d] = -1.0;
                     }
                     Dual3 N, Gn[3];
-                    dual_node<D>(MD, B, i, j, k, rel, N, Gn);
+                    dual_node<D>(MD, B, i, j, k, N, Gn);
                     double u[3] = {};
 #pragma unroll
                     for (int d = 0; d < D; ++d) {

@@ -43,6 +43,24 @@ __device__ __forceinline__ int block_split(const int* totals, int per_cta) {
     return int(s < 1 ? 1 : (s > 8 ? 8 : s));
 }
 
+// CTAs that share one block in a kernel that takes passes of up to `nb` particles
+// and may sum several passes before it adds them to the grid, for `nblk` blocks
+// on a grid of `ctas`: enough for about four pieces per CTA while every piece
+// still has a full pass, and for one piece per CTA where the blocks are fewer than
+// the CTAs (passes of `per` < nb particles then, at least 128). Short passes cost:
+// a 64^3 B-spline block of 262 k particles (512 blocks on 444 CTAs) took 5% longer
+// per step with two half passes per block than with one.
+__device__ __forceinline__ int block_pieces(const int* totals, int nblk, int nb, int ctas, int& per) {
+    per = nb;
+    const int nact = totals[0];
+    if (nact <= 0 || nblk <= 0) return 1;
+    const int avg = int((long long)totals[1] / nact), passes = (avg + nb - 1) / nb;
+    const int full = min(passes, (4 * ctas + nblk - 1) / nblk), fill = min(ctas / nblk, (avg + 127) / 128);
+    const int pieces = max(1, min(8, max(full, fill)));
+    if (pieces > passes) per = min(nb, max(128, ((avg + pieces - 1) / pieces + 7) & ~7));
+    return pieces;
+}
+
 // The passes of one block's particle range [s0, s1) for kernels that hold `per`
 // particles (a multiple of 8) at a time: pass i of count() = ceil(n / per)
 // takes the 8-particle chunks i, i + count(), i + 2 count(), ..., so every pass
@@ -241,17 +259,29 @@ __device__ __forceinline__ void grid_add(const GView<T>& G, const MT& M, int* er
     }
 }
 
+// A particle's uGIMP length over the spacing: in the state type, its inverse,
+// and in FP64 (for the windows of the FP64-position form).
+template <class T>
+struct GimpLen {
+    T ln, il;
+    double ln64;
+};
+
 // Step scalars, converted once to the state type.
 template <class T>
 struct Scalars {
     T dt, mass, V0, g[3], gimp_l, alpha;
     double dt64, V0_64, mu, lam, hardening, yield_stress;
+    GimpLen<T> gimp;  // of gimp_l, for all particles when none has its own
     int basis, transfer, material, wall_mask, wall_layers;
 };
 
 template <class T>
-inline Scalars<T> make_scalars(const tb_step_params& p) {
+inline Scalars<T> make_scalars(const tb_step_params& p, const tb_mesh& m) {
     Scalars<T> s{};
+    s.gimp.ln = T(p.gimp_l) / T(m.h);
+    s.gimp.il = T(1) / s.gimp.ln;
+    s.gimp.ln64 = double(T(p.gimp_l)) / m.h;
     s.dt = T(p.dt);
     s.mass = T(p.mass);
     s.V0 = T(p.V0);
@@ -348,20 +378,39 @@ __device__ __forceinline__ void jet_bspline_quadratic(T xi, T& val, T& der) {
     }
 }
 
+// a / l given il = 1 / l: the product, corrected once by its residual a - q l
+// (the final quotient step of P. Markstein, IBM J. Res. Dev. 34, 1990), so that a
+// length shared by all particles does not put the rounding of its inverse into
+// every weight.
+__device__ __forceinline__ float quotient(float a, float l, float il) {
+    const float q = a * il;
+    return fmaf(fmaf(-q, l, a), il, q);
+}
+__device__ __forceinline__ double quotient(double a, double l, double il) {
+    const double q = a * il;
+    return fma(fma(-q, l, a), il, q);
+}
+__device__ __forceinline__ Dual3 quotient(const Dual3& a, const Dual3& l, const Dual3&) { return a / l; }
+
+// uGIMP jets (gimp.jl:16-40); il = 1 / l, computed once per particle or per scene.
+// (The nine jets of a 3D particle held 27 divisions by l, about half of the
+// instructions of the WLS(uGIMP) kernels' basis.)
 template <class T>
-__device__ __forceinline__ void jet_ugimp(T xi, T l, T& val, T& der) {
+__device__ __forceinline__ void jet_ugimp(T xi, T l, T il, T& val, T& der) {
     T s = signbit(xi) ? T(-1) : T(1);
     T a = fabs(xi);
-    if (a < l / T(2)) {
-        val = T(1) - (T(4) * (a * a) + l * l) / (T(4) * l);
-        der = -(T(2) * a / l) * s;
-    } else if (a < T(1) - l / T(2)) {
+    const T hl = l * T(0.5);
+    if (a < hl) {
+        val = T(1) - quotient(a * a + hl * hl, l, il);
+        der = -quotient(T(2) * a, l, il) * s;
+    } else if (a < T(1) - hl) {
         val = T(1) - a;
         der = -s;
-    } else if (a < T(1) + l / T(2)) {
-        T t = T(1) + l / T(2) - a;
-        val = (t * t) / (T(2) * l);
-        der = -(t / l) * s;
+    } else if (a < T(1) + hl) {
+        T t = T(1) + hl - a;
+        const T q = quotient(t, l, il);
+        val = T(0.5) * (t * q);
+        der = -q * s;
     } else {
         val = T(0);
         der = T(0);
@@ -396,7 +445,7 @@ __device__ __forceinline__ void bspline_quadratic_axis(T xi, T* v0, T* v1) {
 // cartesian.jl:190-199). Returns false when the particle is outside the mesh.
 template <int D, class T>
 __device__ __forceinline__ bool axis_window(const DMesh<D, T>& M, int basis, const T* x, T lnorm, T* xi, int* lo,
-                                            int* cnt) {
+                                            int* cnt, bool* cut = nullptr) {
     bool inside = true;
 #pragma unroll
     for (int d = 0; d < D; ++d) {
@@ -419,16 +468,17 @@ __device__ __forceinline__ bool axis_window(const DMesh<D, T>& M, int basis, con
         }
         lo[d] = max(s, 0);
         cnt[d] = min(e, M.n[d] - 1) - lo[d] + 1;
+        if (cut) cut[d] = s < 0 || e > M.n[d] - 1;  // the mesh cuts the support on this axis
     }
     return true;
 }
 
 template <int D, class T>
-__device__ __forceinline__ bool axis_weights(const DMesh<D, T>& M, int basis, const T* x, T lnorm, Axis<T>* ax,
-                                             bool& full) {
+__device__ __forceinline__ bool axis_weights(const DMesh<D, T>& M, int basis, const T* x, const GimpLen<T>& gl,
+                                             Axis<T>* ax, bool& full, bool* cut = nullptr) {
     T xi[3];
     int lo[3], cnt[3];
-    if (!axis_window<D, T>(M, basis, x, lnorm, xi, lo, cnt)) return false;
+    if (!axis_window<D, T>(M, basis, x, gl.ln, xi, lo, cnt, cut)) return false;
     const bool gimp = basis_is_gimp(basis);
     full = true;
 #pragma unroll
@@ -450,7 +500,7 @@ __device__ __forceinline__ bool axis_weights(const DMesh<D, T>& M, int basis, co
             ax[d].der[k] = T(0);
             if (k < ax[d].cnt) {
                 T xn = (x[d] - node_coord(M, d, ax[d].lo + k)) * M.h_inv;
-                if (gimp) jet_ugimp(xn, lnorm, ax[d].val[k], ax[d].der[k]);
+                if (gimp) jet_ugimp(xn, gl.ln, gl.il, ax[d].val[k], ax[d].der[k]);
                 else jet_bspline_quadratic(xn, ax[d].val[k], ax[d].der[k]);
             }
         }
@@ -519,113 +569,75 @@ __device__ __forceinline__ void node_weight(const DMesh<D, T>& M, const Axis<T>*
     }
 }
 
-// WLS moment-matrix inverse (wls.jl:51-68); the closed form diag(1, 4/h^2) for a
-// full quadratic B-spline support (wls.jl:29-49). Returns false if singular.
-// `r[d][k]` = X_{lo+k} - x_p on axis d. The kernel weight is a product of axis
-// factors and P = (1, X - x_p) has one axis per component, so
-// M = sum_i w_i P_i P_i^T is built from the axis moments S0 = sum w, S1 = sum w r,
-// S2 = sum w r^2: M00 = prod S0, M0a = S1_a prod_{d!=a} S0_d,
-// Maa = S2_a prod_{d!=a} S0_d, Mab = S1_a S1_b prod_{d!=a,b} S0_d -- the
-// reference's sum over the window's nodes, regrouped (equal to rounding).
-// Slots beyond a truncated window have w = 0 and drop out.
+// WLS weights in closed form. The reference inverts the moment matrix
+// M = sum_i w_i P_i P_i^T, P = (1, X - x_p) (wls.jl:51-68; diag(1, 4/h^2) for a
+// full quadratic B-spline support, wls.jl:29-49). The kernel weight is a product
+// of axis factors and P has one axis per component, so with the axis moments
+//   S0 = sum w,  u = sum w r / S0,  var = sum w (r - u)^2 / S0   (r = X - x_p)
+// M = prod S0 [[1, u^T], [u, diag(var) + u u^T]], whose inverse is known:
+//   grad N_i = G_i,  G_{i,d} = W_i (r_d - u_d) / var_d,   N_i = W_i - u . G_i,
+// W_i = prod w / S0. Per axis the jets become (w / S0, w / S0 (r - u) / var): the
+// weights keep the product form of the plain kernel, and only N needs the
+// correction -u . G. On a support that the mesh does not cut, S0 = 1 and u = 0
+// (the kernels reproduce linear fields) and N_i is the kernel itself; a
+// B-spline's var is h^2/4. `r[d][k]` = X_{lo+k} - x_p; der is stored in units of
+// xi (times h) like the plain jets. False where M is singular.
 template <int D, class T>
-__device__ __forceinline__ bool wls_minv(const DMesh<D, T>& M, const Axis<T>* ax, const T (&r)[3][3], bool closed,
-                                         T (&Mi)[D + 1][D + 1]) {
-    constexpr int N = D + 1;
-#pragma unroll
-    for (int a = 0; a < N; ++a)
-#pragma unroll
-        for (int c = 0; c < N; ++c) Mi[a][c] = T(0);
-    if (closed) {
-        Mi[0][0] = T(1);
-        T cval = T(4) / (M.h * M.h);
-#pragma unroll
-        for (int d = 1; d < N; ++d) Mi[d][d] = cval;
-        return true;
-    }
-    T S0[3], S1[3], S2[3];
+__device__ __forceinline__ bool wls_correct(const DMesh<D, T>& M, bool bspline, const bool* cut, const T (&r)[3][3],
+                                            Axis<T>* ax, T* u, T* var) {
 #pragma unroll
     for (int d = 0; d < D; ++d) {
-        S0[d] = S1[d] = S2[d] = T(0);
+        u[d] = T(0);
+        if (cut[d]) {
+            T S0 = T(0), S1 = T(0);
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const T w = ax[d].val[k];
-            S0[d] += w;
-            S1[d] += w * r[d][k];
-            S2[d] += (w * r[d][k]) * r[d][k];
+            for (int k = 0; k < 3; ++k) {
+                S0 += ax[d].val[k];
+                S1 += ax[d].val[k] * r[d][k];
+            }
+            if (S0 == T(0)) return false;
+            u[d] = S1 / S0;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) ax[d].val[k] = ax[d].val[k] / S0;
         }
+        if (bspline && !cut[d]) {
+            var[d] = M.h * M.h / T(4);
+        } else {
+            var[d] = T(0);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const T q = r[d][k] - u[d];
+                var[d] += ax[d].val[k] * q * q;
+            }
+        }
+        if (var[d] == T(0)) return false;
+        const T c = M.h / var[d];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) ax[d].der[k] = ax[d].val[k] * ((r[d][k] - u[d]) * c);
     }
-    T A[N][2 * N];
-#pragma unroll
-    for (int a = 0; a < N; ++a)
-#pragma unroll
-        for (int c = 0; c < N; ++c) {
-            // factor of axis d in entry (a, c): S2 if both index d, S1 if one does, else S0
-            T v = T(1);
-#pragma unroll
-            for (int d = 0; d < D; ++d) {
-                const int hits = (a == d + 1) + (c == d + 1);
-                v *= hits == 2 ? S2[d] : (hits == 1 ? S1[d] : S0[d]);
-            }
-            A[a][c] = v;
-            A[a][c + N] = (a == c) ? T(1) : T(0);
-        }
-    // Gauss-Jordan with partial pivoting on [M | I].
-#pragma unroll
-    for (int c = 0; c < N; ++c) {
-        int p = c;
-#pragma unroll
-        for (int q = c + 1; q < N; ++q)
-            if (fabs(A[q][c]) > fabs(A[p][c])) p = q;
-        if (A[p][c] == T(0)) return false;
-        if (p != c) {
-#pragma unroll
-            for (int k = 0; k < 2 * N; ++k) {
-                T t = A[p][k];
-                A[p][k] = A[c][k];
-                A[c][k] = t;
-            }
-        }
-        T inv = T(1) / A[c][c];
-#pragma unroll
-        for (int k = 0; k < 2 * N; ++k) A[c][k] *= inv;
-#pragma unroll
-        for (int q = 0; q < N; ++q)
-            if (q != c) {
-                T f = A[q][c];
-#pragma unroll
-                for (int k = 0; k < 2 * N; ++k) A[q][k] -= f * A[c][k];
-            }
-    }
-#pragma unroll
-    for (int a = 0; a < N; ++a)
-#pragma unroll
-        for (int c = 0; c < N; ++c) Mi[a][c] = A[a][c + N];
     return true;
 }
 
 // Basis state of one particle, ready for per-node evaluation in a transfer.
+// WLS: u and var of wls_correct, `cut` if the mesh cuts the support (u != 0).
 template <int D, class T>
 struct Basis {
     Axis<T> ax[D];
-    T Mi[D + 1][D + 1];
-    bool wls;
+    T u[D], var[D];
+    bool wls, cut;
 };
 
 // Prepare the basis of one particle. Returns false for an empty window.
 template <int D, class T, bool ALLOW_WLS = true>
-__device__ __forceinline__ bool prepare_basis(const DMesh<D, T>& M, int basis, const T* x, T l_abs,
+__device__ __forceinline__ bool prepare_basis(const DMesh<D, T>& M, int basis, const T* x, const GimpLen<T>& gl,
                                               Basis<D, T>& B, int* err) {
-    T lnorm = T(0);
-    if (basis_is_gimp(basis)) {
-        lnorm = l_abs / M.h;
-        if (!(lnorm >= T(0) && lnorm <= T(1))) {
-            atomicOr(err, ERR_GIMP_LENGTH);
-            return false;
-        }
+    if (basis_is_gimp(basis) && !(gl.ln >= T(0) && gl.ln <= T(1))) {
+        atomicOr(err, ERR_GIMP_LENGTH);
+        return false;
     }
-    bool full = false;
-    if (!axis_weights<D, T>(M, basis, x, lnorm, B.ax, full)) return false;
+    bool full = false, cut[3];
+    if (!axis_weights<D, T>(M, basis, x, gl, B.ax, full, cut)) return false;
+    B.cut = cut[0] || cut[1] || (D == 3 && cut[2]);
     if (basis_is_kc(basis) && !full) {
         T r[3][3] = {};
 #pragma unroll
@@ -639,15 +651,12 @@ __device__ __forceinline__ bool prepare_basis(const DMesh<D, T>& M, int basis, c
     }
     B.wls = ALLOW_WLS && (basis == TB_WLS_BSPLINE_QUADRATIC || basis == TB_WLS_UGIMP);
     if constexpr (ALLOW_WLS) if (B.wls) {
-        bool closed = (basis == TB_WLS_BSPLINE_QUADRATIC) && full;
         T r[3][3] = {};
-        if (!closed) {
 #pragma unroll
-            for (int d = 0; d < D; ++d)
+        for (int d = 0; d < D; ++d)
 #pragma unroll
-                for (int k = 0; k < 3; ++k) r[d][k] = node_coord(M, d, B.ax[d].lo + k) - x[d];
-        }
-        if (!wls_minv<D, T>(M, B.ax, r, closed, B.Mi)) {
+            for (int k = 0; k < 3; ++k) r[d][k] = node_coord(M, d, B.ax[d].lo + k) - x[d];
+        if (!wls_correct<D, T>(M, basis == TB_WLS_BSPLINE_QUADRATIC, cut, r, B.ax, B.u, B.var)) {
             atomicOr(err, ERR_WLS_SINGULAR);
             return false;
         }
@@ -660,16 +669,15 @@ __device__ __forceinline__ bool prepare_basis(const DMesh<D, T>& M, int basis, c
 // only the offset from the window's first node, a number in [0, 3), is rounded
 // to T before the jets are evaluated, so the weights carry T's relative
 // precision of that offset rather than of the absolute coordinate. Window rules
-// as axis_window (B-spline and uGIMP; WLS is not on this form).
+// as axis_window.
 template <int D, class T>
 __device__ __forceinline__ bool axis_window_x64(const DMesh<D, T>& M, int basis, const double* x, double lnorm,
-                                                double* xi, int* lo, int* cnt) {
+                                                double* xi, int* lo, int* cnt, bool* cut = nullptr) {
     bool inside = true;
 #pragma unroll
     for (int d = 0; d < D; ++d) {
         xi[d] = (x[d] - M.xmin64[d]) * M.h_inv64;
-        const double c = floor(xi[d]);
-        inside = inside && (c >= 0.0 && c <= double(M.n[d] - 2));
+        inside = inside && xi[d] >= 0.0 && xi[d] < double(M.n[d] - 1);  // floor(xi) in [0, n - 2]
     }
     if (!inside) return false;
     const bool gimp = basis_is_gimp(basis);
@@ -686,26 +694,25 @@ __device__ __forceinline__ bool axis_window_x64(const DMesh<D, T>& M, int basis,
         }
         lo[d] = max(st, 0);
         cnt[d] = min(e, M.n[d] - 1) - lo[d] + 1;
+        if (cut) cut[d] = st < 0 || e > M.n[d] - 1;
     }
     return true;
 }
 
 template <int D, class T, bool ALLOW_WLS = false>
-__device__ __forceinline__ bool prepare_basis_x64(const DMesh<D, T>& M, int basis, const double* x, T l_abs,
-                                                  Basis<D, T>& B, int* err) {
-    double lnorm = 0.0;
+__device__ __forceinline__ bool prepare_basis_x64(const DMesh<D, T>& M, int basis, const double* x,
+                                                  const GimpLen<T>& gl, Basis<D, T>& B, int* err) {
     const bool gimp = basis_is_gimp(basis);
-    if (gimp) {
-        lnorm = double(l_abs) / M.h64;
-        if (!(lnorm >= 0.0 && lnorm <= 1.0)) {
-            atomicOr(err, ERR_GIMP_LENGTH);
-            return false;
-        }
+    if (gimp && !(gl.ln64 >= 0.0 && gl.ln64 <= 1.0)) {
+        atomicOr(err, ERR_GIMP_LENGTH);
+        return false;
     }
     double xi[3];
     int lo[3], cnt[3];
-    if (!axis_window_x64<D, T>(M, basis, x, lnorm, xi, lo, cnt)) return false;
-    B.wls = false;
+    bool cut[3];
+    if (!axis_window_x64<D, T>(M, basis, x, gl.ln64, xi, lo, cnt, cut)) return false;
+    B.cut = cut[0] || cut[1] || (D == 3 && cut[2]);
+    B.wls = ALLOW_WLS && (basis == TB_WLS_BSPLINE_QUADRATIC || basis == TB_WLS_UGIMP);
     bool full = true;
 #pragma unroll
     for (int d = 0; d < D; ++d) {
@@ -713,13 +720,6 @@ __device__ __forceinline__ bool prepare_basis_x64(const DMesh<D, T>& M, int basi
         B.ax[d].cnt = cnt[d];
         full = full && cnt[d] == 3;
     }
-    // X_{lo+k} - x_p in FP64, rounded once to T (KernelCorrection and WLS)
-    auto rel = [&](T (&r)[3][3]) {
-#pragma unroll
-        for (int d = 0; d < D; ++d)
-#pragma unroll
-            for (int k = 0; k < 3; ++k) r[d][k] = T(__dadd_rn(M.xmin64[d], __dmul_rn(double(lo[d] + k), M.h64)) - x[d]);
-    };
     if (!gimp && full) {
         // the fast path's t = fract(xi - 1/2) is xi - 1/2 - lo, in [0, 1); kept
         // below 1 after rounding so that the jets stay on the FP64 window
@@ -729,67 +729,59 @@ __device__ __forceinline__ bool prepare_basis_x64(const DMesh<D, T>& M, int basi
             if (t >= T(1)) t = T(1) - T(1) / T(1 << 24);
             bspline_quadratic_poly(t, B.ax[d].val, B.ax[d].der);
         }
-    } else {
-        const T ln = T(lnorm);
+        if (!B.wls) return true;
+    }
+    // offsets xi - (lo + k) of the particle from its window's nodes in FP64,
+    // rounded once to T: the jets' argument and, times -h, X_{lo+k} - x_p
+    T r[3][3] = {};
 #pragma unroll
-        for (int d = 0; d < D; ++d) {
+    for (int d = 0; d < D; ++d) {
+        const double t = xi[d] - double(lo[d]);
+        const T xn[3] = {T(t), T(t - 1.0), T(t - 2.0)};
 #pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                B.ax[d].val[k] = T(0);
-                B.ax[d].der[k] = T(0);
+        for (int k = 0; k < 3; ++k) {
+            r[d][k] = -xn[k] * M.h;
+            if (gimp || !full) {
+                T v = T(0), g = T(0);
                 if (k < cnt[d]) {
-                    const T xn = T(xi[d] - double(lo[d] + k));
-                    if (gimp) jet_ugimp(xn, ln, B.ax[d].val[k], B.ax[d].der[k]);
-                    else jet_bspline_quadratic(xn, B.ax[d].val[k], B.ax[d].der[k]);
+                    if (gimp) jet_ugimp(xn[k], gl.ln, gl.il, v, g);
+                    else jet_bspline_quadratic(xn[k], v, g);
                 }
-            }
-        }
-        if (basis_is_kc(basis) && !full) {
-            T r[3][3] = {};
-            rel(r);
-            if (!kc_correct<D, T>(M, basis == TB_KC_BSPLINE_QUADRATIC, r, B.ax)) {
-                atomicOr(err, ERR_WLS_SINGULAR);
-                return false;
+                B.ax[d].val[k] = v;
+                B.ax[d].der[k] = g;
             }
         }
     }
-    if constexpr (ALLOW_WLS) {
-        B.wls = basis == TB_WLS_BSPLINE_QUADRATIC || basis == TB_WLS_UGIMP;
-        if (B.wls) {
-            const bool closed = basis == TB_WLS_BSPLINE_QUADRATIC && full;
-            T r[3][3] = {};
-            if (!closed) rel(r);
-            if (!wls_minv<D, T>(M, B.ax, r, closed, B.Mi)) {
-                atomicOr(err, ERR_WLS_SINGULAR);
-                return false;
-            }
-        }
+    bool ok = true;
+    if (basis_is_kc(basis)) {
+        if (!full) ok = kc_correct<D, T>(M, basis == TB_KC_BSPLINE_QUADRATIC, r, B.ax);
+    } else if constexpr (ALLOW_WLS) {
+        if (B.wls) ok = wls_correct<D, T>(M, basis == TB_WLS_BSPLINE_QUADRATIC, cut, r, B.ax, B.u, B.var);
     }
-    return true;
+    if (!ok) atomicOr(err, ERR_WLS_SINGULAR);
+    return ok;
 }
 
-// w and grad w at window slot (i, j, k); `rel` = X_i - x_p per axis.
+// The uGIMP length of particle p (its own, or the scene's).
 template <int D, class T>
-__device__ __forceinline__ void eval_node(const DMesh<D, T>& M, const Basis<D, T>& B, int i, int j, int k,
-                                          const T* rel, T& w, T* dw) {
+__device__ __forceinline__ GimpLen<T> gimp_len(const DMesh<D, T>& M, const PView<T>& P, const Scalars<T>& s, long long p) {
+    if (!P.l) return s.gimp;
+    GimpLen<T> g;
+    const T l = P.l[p];
+    g.ln = l / M.h;
+    g.il = T(1) / g.ln;
+    g.ln64 = double(l) / M.h64;
+    return g;
+}
+
+// w and grad w at window slot (i, j, k).
+template <int D, class T>
+__device__ __forceinline__ void eval_node(const DMesh<D, T>& M, const Basis<D, T>& B, int i, int j, int k, T& w,
+                                          T* dw) {
     node_weight<D, T>(M, B.ax, i, j, k, w, dw);
     if (B.wls) {
-        constexpr int N = D + 1;
-        T P[N];
-        P[0] = T(1);
 #pragma unroll
-        for (int d = 0; d < D; ++d) P[d + 1] = rel[d];
-        T wq[N];
-#pragma unroll
-        for (int r = 0; r < N; ++r) {
-            T acc = T(0);
-#pragma unroll
-            for (int c = 0; c < N; ++c) acc += B.Mi[r][c] * P[c];
-            wq[r] = w * acc;
-        }
-        w = wq[0];
-#pragma unroll
-        for (int d = 0; d < D; ++d) dw[d] = wq[d + 1];
+        for (int d = 0; d < D; ++d) w -= B.u[d] * dw[d];
     }
 }
 

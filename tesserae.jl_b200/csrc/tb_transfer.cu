@@ -238,38 +238,61 @@ __device__ __forceinline__ void g2p_finish(const PView<T>& P, const Scalars<T>& 
     particle_update<D, T, VM>(P, s, p, gv, F);
 }
 
-template <int D, class T, int BW, bool GEN, bool X64, bool VM = false>
-__global__ void __launch_bounds__(128, (GEN || VM) ? (sizeof(T) == 4 ? 4 : 2) : (sizeof(T) == 4 ? 8 : 4)) g2p_tile_kernel(DMesh<D, T> M, GView<T> G, PView<T> P, Scalars<T> s,
+// GEN: which basis and transfer the kernel gathers for.
+//   G_PLAIN    B-spline / uGIMP / KernelCorrection, FLIP/PIC: separable contraction
+//   G_WLS      WLS, FLIP/PIC: the same contraction with the WLS jets (wls_correct).
+//              N_i = W_i on a window that the mesh does not cut; a cut window
+//              takes the per-node loop (N_i = W_i - u . G_i)
+//   G_WLS_APIC WLS, APIC: as G_WLS; sum N v (x) r = grad_v diag(var) comes without
+//              another sum, since G_{i,d} = W_i r_d / var_d
+//   G_APIC     plain kernel, APIC: the contraction with the first moments of r
+// Before the closed form every WLS / APIC particle evaluated a (D+1)^2 moment
+// inverse at each of its nodes: dam break at half resolution, 18.2 M particles,
+// FP32 with FP64 positions, 3.66 ms; 1.83 ms now.
+enum : int { G_PLAIN = 0, G_WLS = 1, G_WLS_APIC = 2, G_APIC = 3 };
+
+// CTAs of 128 threads per SM. General kinds in FP32: 6 (80 registers) measured 1.92
+// ms on the dam break below, 4 / 5 / 8: 2.01 / 2.28 / 2.10 ms.
+constexpr int g2p_ctas(int gen, bool vm, bool fp32) {
+    if (vm) return fp32 ? 4 : 2;
+    if (gen != G_PLAIN) return fp32 ? 6 : 3;
+    return fp32 ? 8 : 4;
+}
+
+template <int D, class T, int BW, int GEN, bool X64, bool VM = false>
+__global__ void __launch_bounds__(128, g2p_ctas(GEN, VM, sizeof(T) == 4)) g2p_tile_kernel(DMesh<D, T> M, GView<T> G, PView<T> P, Scalars<T> s,
                                                        const int* __restrict__ totals,
                                                        const int* __restrict__ blocklist,
                                                        const int* __restrict__ offsets,
                                                        const int* __restrict__ perm, int* err,
                                                        int* __restrict__ next_bid, int* __restrict__ next_count) {
     constexpr int TS = Tile<D, BW>::TS, TN = Tile<D, BW>::TN;
+    constexpr bool WLS = GEN == G_WLS || GEN == G_WLS_APIC, APIC = GEN == G_WLS_APIC || GEN == G_APIC;
     // 3D FP32: node-major, (v_x, v_y, v_z, dv_x) as a float4 at [t] and (dv_y, dv_z)
     // as a float2 after the TN float4s, dv = v - vn: two vector loads per node,
     // whose halves feed packed FP32x2 FMAs. Otherwise component-major: v_r at
     // [r TN + t], dv_r at [(D + r) TN + t]; lanes reading different nodes hit
-    // different banks.
+    // different banks. APIC reads no vn: the tile holds v alone.
     constexpr bool VEC = (D == 3 && sizeof(T) == 4);
-    __shared__ __align__(16) T tile[2 * D * TN];
+    __shared__ __align__(16) T tile[APIC ? (VEC ? 4 : D) * TN : 2 * D * TN];
     auto node_vals = [&](int t, T (&vi)[3], T (&dvi)[3]) {
         if constexpr (VEC) {
             const float4 a = reinterpret_cast<const float4*>(tile)[t];
-            const float2 c = reinterpret_cast<const float2*>(tile + 4 * TN)[t];
             vi[0] = a.x; vi[1] = a.y; vi[2] = a.z;
-            dvi[0] = a.w; dvi[1] = c.x; dvi[2] = c.y;
+            if constexpr (!APIC) {
+                const float2 c = reinterpret_cast<const float2*>(tile + 4 * TN)[t];
+                dvi[0] = a.w; dvi[1] = c.x; dvi[2] = c.y;
+            }
         } else {
 #pragma unroll
             for (int d = 0; d < D; ++d) {
                 vi[d] = tile[d * TN + t];
-                dvi[d] = tile[(D + d) * TN + t];
+                if constexpr (!APIC) dvi[d] = tile[(D + d) * TN + t];
             }
         }
     };
     const int nactive = totals[0];
     const int tid = threadIdx.x, nth = blockDim.x;
-    const bool apic = s.transfer == TB_TRANSFER_APIC;
     // CTA `piece` of `split` sharing a block takes its particles piece nth + tid,
     // (piece + split) nth + tid, ... (block_split: 4 particles per thread)
     const int split = block_split(totals, 4 * nth);
@@ -303,17 +326,19 @@ __global__ void __launch_bounds__(128, (GEN || VM) ? (sizeof(T) == 4 ? 4 : 2) : 
 #pragma unroll
             for (int d = 0; d < D; ++d) {
                 vi[d] = sl >= 0 ? G.v[d][sl] : T(0);
-                const T vni = sl >= 0 ? G.vn[d][sl] : T(0);
-                dvi[d] = vi[d] - vni;
+                if constexpr (!APIC) {
+                    const T vni = sl >= 0 ? G.vn[d][sl] : T(0);
+                    dvi[d] = vi[d] - vni;
+                }
             }
             if constexpr (VEC) {
                 reinterpret_cast<float4*>(tile)[t] = make_float4(vi[0], vi[1], vi[2], dvi[0]);
-                reinterpret_cast<float2*>(tile + 4 * TN)[t] = make_float2(dvi[1], dvi[2]);
+                if constexpr (!APIC) reinterpret_cast<float2*>(tile + 4 * TN)[t] = make_float2(dvi[1], dvi[2]);
             } else {
 #pragma unroll
                 for (int d = 0; d < D; ++d) {
                     tile[d * TN + t] = vi[d];
-                    tile[(D + d) * TN + t] = dvi[d];
+                    if constexpr (!APIC) tile[(D + d) * TN + t] = dvi[d];
                 }
             }
         }
@@ -331,21 +356,20 @@ __global__ void __launch_bounds__(128, (GEN || VM) ? (sizeof(T) == 4 ? 4 : 2) : 
             }
 #pragma unroll
             for (int d = 0; d < D; ++d) vp[d] = P.v[d][p];
-            // F (72 bytes in FP64): the FP32 B-spline/uGIMP kernel (64 registers)
-            // loads it after the gather, where holding it across the gather cost
-            // spills (G2P 1.032 -> 1.019 ms on cube3d); the FP64 and WLS/APIC
-            // kernels load it here so that the load overlaps the gather (loading
-            // it late measured 7% and 1% slower there).
-            constexpr bool LATE_F = !GEN && sizeof(T) == 4;
+            // F (72 bytes in FP64): the FP32 kernels (64 to 80 registers) load it
+            // after the gather, where holding it across the gather cost spills
+            // (G2P 1.032 -> 1.019 ms on cube3d); the FP64 kernels load it here so
+            // that the load overlaps the gather (loading it late measured 7% slower).
+            constexpr bool LATE_F = sizeof(T) == 4;
             double F[3][3];
             if constexpr (!LATE_F) load_F<D, T>(P, p, F);
-            const T l = P.l ? P.l[p] : s.gimp_l;
+            const GimpLen<T> l = gimp_len(M, P, s, p);
             T vpic[3] = {T(0), T(0), T(0)}, dvf[3] = {T(0), T(0), T(0)}, dxs[3] = {T(0), T(0), T(0)};
             T gv[3][3] = {}, Bn[3][3] = {};
             Basis<D, T> B;
             bool in;
-            if constexpr (X64) in = prepare_basis_x64<D, T, GEN>(M, s.basis, xd, l, B, err);
-            else in = prepare_basis<D, T, GEN>(M, s.basis, x, l, B, err);
+            if constexpr (X64) in = prepare_basis_x64<D, T, WLS>(M, s.basis, xd, l, B, err);
+            else in = prepare_basis<D, T, WLS>(M, s.basis, x, l, B, err);
             if (in) {
                 int q0[3] = {0, 0, 0};
                 bool ok = true;
@@ -356,7 +380,115 @@ __global__ void __launch_bounds__(128, (GEN || VM) ? (sizeof(T) == 4 ? 4 : 2) : 
                 }
                 if (!ok) {
                     atomicOr(err, ERR_TILE_RANGE);
-                } else if constexpr (!GEN && VEC) {
+                } else if (WLS && B.cut) {
+                    // a WLS window that the mesh cuts: per-node weights
+#pragma unroll
+                    for (int k = 0; k < (D == 3 ? 3 : 1); ++k)
+#pragma unroll
+                        for (int jj = 0; jj < 3; ++jj)
+#pragma unroll
+                            for (int i = 0; i < 3; ++i) {
+                                const int idx[3] = {i, jj, k};
+                                const int t = (D == 3) ? (q0[0] + i) + TS * ((q0[1] + jj) + TS * (q0[D - 1] + k))
+                                                       : (q0[0] + i) + TS * (q0[1] + jj);
+                                T w, dw[3];
+                                eval_node<D, T>(M, B, i, jj, k, w, dw);
+                                T vi[3], dvi[3];
+                                node_vals(t, vi, dvi);
+#pragma unroll
+                                for (int r = 0; r < D; ++r) {
+                                    vpic[r] += w * vi[r];
+                                    if constexpr (!APIC) dvf[r] += w * dvi[r];
+#pragma unroll
+                                    for (int c = 0; c < D; ++c) gv[r][c] += vi[r] * dw[c];
+                                }
+                                if constexpr (APIC) {
+#pragma unroll
+                                    for (int c = 0; c < D; ++c) {
+                                        T rel;
+                                        if constexpr (X64)  // X_i - x_p in FP64, rounded once
+                                            rel = T(__dadd_rn(M.xmin64[c], __dmul_rn(double(B.ax[c].lo + idx[c]), M.h64)) -
+                                                    xd[c]);
+                                        else
+                                            rel = node_coord(M, c, B.ax[c].lo + idx[c]) - x[c];
+#pragma unroll
+                                        for (int r = 0; r < D; ++r) Bn[r][c] += (w * vi[r]) * rel;
+                                    }
+                                }
+                            }
+                } else if constexpr (APIC && VEC) {
+                    float gx[3], rr[3][3];
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) gx[i] = B.ax[0].der[i] * M.h_inv;
+                    if constexpr (GEN == G_APIC) {
+#pragma unroll
+                        for (int d = 0; d < 3; ++d)
+#pragma unroll
+                            for (int k = 0; k < 3; ++k) {
+                                if constexpr (X64)
+                                    rr[d][k] = float(__dadd_rn(M.xmin64[d], __dmul_rn(double(B.ax[d].lo + k), M.h64)) - xd[d]);
+                                else
+                                    rr[d][k] = node_coord(M, d, B.ax[d].lo + k) - x[d];
+                            }
+                    }
+                    const float4* tA = reinterpret_cast<const float4*>(tile);
+                    const float2 z2 = make_float2(0.f, 0.f);
+                    float2 p01 = z2, g0 = z2, g1 = z2, g2 = z2, b0 = z2, b1 = z2, b2 = z2;
+                    float pz = 0.f, g0z = 0.f, g1z = 0.f, g2z = 0.f, b0z = 0.f, b1z = 0.f, b2z = 0.f;
+#pragma unroll
+                    for (int k = 0; k < 3; ++k)
+#pragma unroll
+                        for (int jj = 0; jj < 3; ++jj) {
+                            float2 A01 = z2, G01 = z2, R01 = z2;
+                            float Az = 0.f, Gz = 0.f, Rz = 0.f;
+                            const int t0 = q0[0] + TS * ((q0[1] + jj) + TS * (q0[2] + k));
+#pragma unroll
+                            for (int i = 0; i < 3; ++i) {
+                                const float4 a = tA[t0 + i];
+                                const float wx = B.ax[0].val[i];
+                                const float2 v01 = make_float2(a.x, a.y);
+                                A01 = __ffma2_rn(make_float2(wx, wx), v01, A01);
+                                Az = __fmaf_rn(wx, a.z, Az);
+                                G01 = __ffma2_rn(make_float2(gx[i], gx[i]), v01, G01);
+                                Gz = __fmaf_rn(gx[i], a.z, Gz);
+                                if constexpr (GEN == G_APIC) {
+                                    const float wr = wx * rr[0][i];
+                                    R01 = __ffma2_rn(make_float2(wr, wr), v01, R01);
+                                    Rz = __fmaf_rn(wr, a.z, Rz);
+                                }
+                            }
+                            const float wyz = B.ax[1].val[jj] * B.ax[2].val[k];
+                            const float dyz = (B.ax[1].der[jj] * M.h_inv) * B.ax[2].val[k];
+                            const float wdz = B.ax[1].val[jj] * (B.ax[2].der[k] * M.h_inv);
+                            const float2 W = make_float2(wyz, wyz);
+                            p01 = __ffma2_rn(W, A01, p01);
+                            pz = __fmaf_rn(wyz, Az, pz);
+                            g0 = __ffma2_rn(W, G01, g0);
+                            g0z = __fmaf_rn(wyz, Gz, g0z);
+                            g1 = __ffma2_rn(make_float2(dyz, dyz), A01, g1);
+                            g1z = __fmaf_rn(dyz, Az, g1z);
+                            g2 = __ffma2_rn(make_float2(wdz, wdz), A01, g2);
+                            g2z = __fmaf_rn(wdz, Az, g2z);
+                            if constexpr (GEN == G_APIC) {
+                                const float wry = wyz * rr[1][jj], wrz = wyz * rr[2][k];
+                                b0 = __ffma2_rn(W, R01, b0);
+                                b0z = __fmaf_rn(wyz, Rz, b0z);
+                                b1 = __ffma2_rn(make_float2(wry, wry), A01, b1);
+                                b1z = __fmaf_rn(wry, Az, b1z);
+                                b2 = __ffma2_rn(make_float2(wrz, wrz), A01, b2);
+                                b2z = __fmaf_rn(wrz, Az, b2z);
+                            }
+                        }
+                    vpic[0] = p01.x; vpic[1] = p01.y; vpic[2] = pz;
+                    gv[0][0] = g0.x; gv[1][0] = g0.y; gv[2][0] = g0z;
+                    gv[0][1] = g1.x; gv[1][1] = g1.y; gv[2][1] = g1z;
+                    gv[0][2] = g2.x; gv[1][2] = g2.y; gv[2][2] = g2z;
+                    if constexpr (GEN == G_APIC) {
+                        Bn[0][0] = b0.x; Bn[1][0] = b0.y; Bn[2][0] = b0z;
+                        Bn[0][1] = b1.x; Bn[1][1] = b1.y; Bn[2][1] = b1z;
+                        Bn[0][2] = b2.x; Bn[1][2] = b2.y; Bn[2][2] = b2z;
+                    }
+                } else if constexpr (VEC) {
                     // The separable contraction below with the component pairs of the
                     // node-major tile in packed FP32x2 FMAs; every lane of a pair is
                     // the scalar form's FMA with the same operands in the same order.
@@ -409,19 +541,29 @@ __global__ void __launch_bounds__(128, (GEN || VM) ? (sizeof(T) == 4 ? 4 : 2) : 
                     gv[0][0] = g0.x; gv[1][0] = g0.y; gv[2][0] = g0z;
                     gv[0][1] = g1.x; gv[1][1] = g1.y; gv[2][1] = g1z;
                     gv[0][2] = g2.x; gv[1][2] = g2.y; gv[2][2] = g2z;
-#pragma unroll
-                    for (int d = 0; d < D; ++d) dxs[d] = vpic[d] * s.dt;
-                } else if constexpr (!GEN) {
+                } else {
                     // Separable contraction: sum over the x-slot first, then weight
                     // the partial sums with the y (and z) factors.
-                    T dxh[3];
+                    T dxh[3], rr[3][3] = {};
 #pragma unroll
                     for (int i = 0; i < 3; ++i) dxh[i] = B.ax[0].der[i] * M.h_inv;
+                    if constexpr (GEN == G_APIC) {
+#pragma unroll
+                        for (int d = 0; d < D; ++d)
+#pragma unroll
+                            for (int k = 0; k < 3; ++k) {
+                                if constexpr (X64)
+                                    rr[d][k] = T(__dadd_rn(M.xmin64[d], __dmul_rn(double(B.ax[d].lo + k), M.h64)) - xd[d]);
+                                else
+                                    rr[d][k] = node_coord(M, d, B.ax[d].lo + k) - x[d];
+                            }
+                    }
 #pragma unroll
                     for (int k = 0; k < (D == 3 ? 3 : 1); ++k)
 #pragma unroll
                         for (int jj = 0; jj < 3; ++jj) {
                             T Av[3] = {T(0), T(0), T(0)}, Adv[3] = {T(0), T(0), T(0)}, Ag[3] = {T(0), T(0), T(0)};
+                            T Ar[3] = {T(0), T(0), T(0)};
                             const int t0 = (D == 3) ? q0[0] + TS * ((q0[1] + jj) + TS * (q0[D - 1] + k))
                                                     : q0[0] + TS * (q0[1] + jj);
 #pragma unroll
@@ -430,10 +572,11 @@ __global__ void __launch_bounds__(128, (GEN || VM) ? (sizeof(T) == 4 ? 4 : 2) : 
                                 const T wx = B.ax[0].val[i], gx = dxh[i];
 #pragma unroll
                                 for (int r = 0; r < D; ++r) {
-                                    const T vi = nd[r * TN], dvi = nd[(D + r) * TN];
+                                    const T vi = nd[r * TN];
                                     Av[r] += wx * vi;
-                                    Adv[r] += wx * dvi;
+                                    if constexpr (!APIC) Adv[r] += wx * nd[(D + r) * TN];
                                     Ag[r] += gx * vi;
+                                    if constexpr (GEN == G_APIC) Ar[r] += (wx * rr[0][i]) * vi;
                                 }
                             }
                             T wyz, dyz, wdz;
@@ -449,56 +592,28 @@ __global__ void __launch_bounds__(128, (GEN || VM) ? (sizeof(T) == 4 ? 4 : 2) : 
 #pragma unroll
                             for (int r = 0; r < D; ++r) {
                                 vpic[r] += wyz * Av[r];
-                                dvf[r] += wyz * Adv[r];
+                                if constexpr (!APIC) dvf[r] += wyz * Adv[r];
                                 gv[r][0] += wyz * Ag[r];
                                 gv[r][1] += dyz * Av[r];
                                 if constexpr (D == 3) gv[r][2] += wdz * Av[r];
+                                if constexpr (GEN == G_APIC) {
+                                    Bn[r][0] += wyz * Ar[r];
+                                    Bn[r][1] += (wyz * rr[1][jj]) * Av[r];
+                                    if constexpr (D == 3) Bn[r][2] += (wyz * rr[2][k]) * Av[r];
+                                }
                             }
                         }
-#pragma unroll
-                    for (int d = 0; d < D; ++d) dxs[d] = vpic[d] * s.dt;
-                } else {
-                    // WLS / APIC: node weights are not separable; per-node loop.
-#pragma unroll
-                    for (int k = 0; k < (D == 3 ? 3 : 1); ++k)
-#pragma unroll
-                        for (int jj = 0; jj < 3; ++jj)
-#pragma unroll
-                            for (int i = 0; i < 3; ++i) {
-                                const int idx[3] = {i, jj, k};
-                                const int t = (D == 3) ? (q0[0] + i) + TS * ((q0[1] + jj) + TS * (q0[D - 1] + k))
-                                                       : (q0[0] + i) + TS * (q0[1] + jj);
-                                T rel[3] = {T(0), T(0), T(0)};
-#pragma unroll
-                                for (int d = 0; d < D; ++d) {
-                                    if constexpr (X64)  // X_i - x_p in FP64, rounded once
-                                        rel[d] = T(__dadd_rn(M.xmin64[d], __dmul_rn(double(B.ax[d].lo + idx[d]), M.h64)) -
-                                                   xd[d]);
-                                    else
-                                        rel[d] = node_coord(M, d, B.ax[d].lo + idx[d]) - x[d];
-                                }
-                                T w, dw[3];
-                                eval_node<D, T>(M, B, i, jj, k, rel, w, dw);
-                                T vi[3], dvi[3];
-                                node_vals(t, vi, dvi);
-#pragma unroll
-                                for (int d = 0; d < D; ++d) {
-                                    vpic[d] += w * vi[d];
-                                    dvf[d] += w * dvi[d];
-                                    dxs[d] += (w * vi[d]) * s.dt;
-                                }
-#pragma unroll
-                                for (int r = 0; r < D; ++r)
-#pragma unroll
-                                    for (int c = 0; c < D; ++c) gv[r][c] += vi[r] * dw[c];
-                                if (apic) {
-#pragma unroll
-                                    for (int r = 0; r < D; ++r)
-#pragma unroll
-                                        for (int c = 0; c < D; ++c) Bn[r][c] += (w * vi[r]) * rel[c];
-                                }
-                            }
                 }
+                if constexpr (GEN == G_WLS_APIC) {
+                    if (!B.cut) {
+#pragma unroll
+                        for (int r = 0; r < D; ++r)
+#pragma unroll
+                            for (int c = 0; c < D; ++c) Bn[r][c] = gv[r][c] * B.var[c];
+                    }
+                }
+#pragma unroll
+                for (int d = 0; d < D; ++d) dxs[d] = vpic[d] * s.dt;
             }
             if constexpr (LATE_F) load_F<D, T>(P, p, F);
             g2p_finish<D, T, VM>(P, s, p, x, vp, vpic, dvf, gv, dxs, Bn, F);
@@ -544,12 +659,11 @@ __global__ void __launch_bounds__(128) g2p_direct_kernel(DMesh<D, T> M, GView<T>
         for (int d = 0; d < D; ++d) vp[d] = P.v[d][p];
         double F[3][3];
         load_F<D, T>(P, p, F);
-        const T l = P.l ? P.l[p] : s.gimp_l;
+        const GimpLen<T> l = gimp_len(M, P, s, p);
         T vpic[3] = {T(0), T(0), T(0)}, dvf[3] = {T(0), T(0), T(0)}, dxs[3] = {T(0), T(0), T(0)};
         T gv[3][3] = {}, Bn[3][3] = {};
         Basis<D, T> B;
         if (prepare_basis<D, T>(M, s.basis, x, l, B, err)) {
-            const bool need_rel = B.wls || apic;
 #pragma unroll
             for (int k = 0; k < (D == 3 ? 3 : 1); ++k)
 #pragma unroll
@@ -567,12 +681,12 @@ __global__ void __launch_bounds__(128) g2p_direct_kernel(DMesh<D, T> M, GView<T>
                             valid = lin >= 0;
                         }
                         T rel[3] = {T(0), T(0), T(0)};
-                        if (need_rel) {
+                        if (apic) {
 #pragma unroll
                             for (int d = 0; d < D; ++d) rel[d] = node_coord(M, d, B.ax[d].lo + idx[d]) - x[d];
                         }
                         T w, dw[3];
-                        eval_node<D, T>(M, B, i, jj, k, rel, w, dw);
+                        eval_node<D, T>(M, B, i, jj, k, w, dw);
                         T vi[3];
 #pragma unroll
                         for (int d = 0; d < D; ++d) {
@@ -650,20 +764,14 @@ __global__ void __launch_bounds__(128) update_weights_kernel(DMesh<D, T> M, PVie
     for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < P.n; p += (long long)gridDim.x * blockDim.x) {
         T x[3];
         load_x<D, T>(P, p, x);
-        const T l = P.l ? P.l[p] : s.gimp_l;
+        const GimpLen<T> l = gimp_len(M, P, s, p);
         Basis<D, T> B;
         const bool ok = prepare_basis<D, T>(M, s.basis, x, l, B, err);
         for (int slot = 0; slot < NW; ++slot) {
             const int i = slot % 3, jj = (slot / 3) % 3, k = slot / 9;
             T w = T(0), dw[3] = {T(0), T(0), T(0)};
             if (ok && i < B.ax[0].cnt && jj < B.ax[1].cnt && (D == 2 || k < B.ax[D - 1].cnt)) {
-                const int idx[3] = {i, jj, k};
-                T rel[3] = {T(0), T(0), T(0)};
-                if (B.wls) {
-#pragma unroll
-                    for (int d = 0; d < D; ++d) rel[d] = node_coord(M, d, B.ax[d].lo + idx[d]) - x[d];
-                }
-                eval_node<D, T>(M, B, i, jj, k, rel, w, dw);
+                eval_node<D, T>(M, B, i, jj, k, w, dw);
             }
             w_out[p * NW + slot] = w;
 #pragma unroll
@@ -706,24 +814,19 @@ cudaError_t launch_grid_update(const DMesh<D, T>& M, const GView<T>& G, const Sc
     return cudaGetLastError();
 }
 
-template <int D, class T, int BW>
-cudaError_t launch_g2p(const DMesh<D, T>& M, const GView<T>& G, const PView<T>& P, const Scalars<T>& s,
-                       const BinBuffers& b, const LaunchCfg& cfg, bool count_next) {
-    if (P.n == 0) return cudaSuccess;
-    const bool gen = s.transfer == TB_TRANSFER_APIC || s.basis == TB_WLS_BSPLINE_QUADRATIC || s.basis == TB_WLS_UGIMP;
-    auto kern = gen ? g2p_tile_kernel<D, T, BW, true, false> : g2p_tile_kernel<D, T, BW, false, false>;
-    const bool vm = s.material == TB_MATERIAL_VONMISES;  // 3D only (checked by the caller)
+template <int D, class T, int BW, int GEN>
+cudaError_t launch_g2p_kind(const DMesh<D, T>& M, const GView<T>& G, const PView<T>& P, const Scalars<T>& s,
+                            const BinBuffers& b, const LaunchCfg& cfg, bool count_next, bool x64, bool vm) {
+    auto kern = g2p_tile_kernel<D, T, BW, GEN, false>;
     if constexpr (D == 3) {
-        if (vm) kern = gen ? g2p_tile_kernel<D, T, BW, true, false, true> : g2p_tile_kernel<D, T, BW, false, false, true>;
+        if (vm) kern = g2p_tile_kernel<D, T, BW, GEN, false, true>;
     }
-    if (P.x64[0]) {  // FP64-position form: FP32 state only (checked by the caller)
-        if constexpr (sizeof(T) == 4) {
-            kern = gen ? g2p_tile_kernel<D, T, BW, true, true> : g2p_tile_kernel<D, T, BW, false, true>;
+    if constexpr (sizeof(T) == 4) {
+        if (x64) {
+            kern = g2p_tile_kernel<D, T, BW, GEN, true>;
             if constexpr (D == 3) {
-                if (vm) kern = gen ? g2p_tile_kernel<D, T, BW, true, true, true> : g2p_tile_kernel<D, T, BW, false, true, true>;
+                if (vm) kern = g2p_tile_kernel<D, T, BW, GEN, true, true>;
             }
-        } else {
-            return cudaErrorInvalidValue;
         }
     }
     const int grid = std::min(occupancy_grid(kern, 128, cfg.num_sms), 8 * M.nblocks);  // blocks may be split
@@ -745,6 +848,21 @@ cudaError_t launch_g2p(const DMesh<D, T>& M, const GView<T>& G, const PView<T>& 
                                        count_next ? b.blockids : nullptr, count_next ? b.counts : nullptr);
     *cfg.launches += 2;
     return cudaGetLastError();
+}
+
+template <int D, class T, int BW>
+cudaError_t launch_g2p(const DMesh<D, T>& M, const GView<T>& G, const PView<T>& P, const Scalars<T>& s,
+                       const BinBuffers& b, const LaunchCfg& cfg, bool count_next) {
+    if (P.n == 0) return cudaSuccess;
+    const bool wls = s.basis == TB_WLS_BSPLINE_QUADRATIC || s.basis == TB_WLS_UGIMP;
+    const bool apic = s.transfer == TB_TRANSFER_APIC;
+    const bool vm = s.material == TB_MATERIAL_VONMISES;  // 3D only (checked by the caller)
+    const bool x64 = P.x64[0] != nullptr;  // FP64-position form: FP32 state only (checked by the caller)
+    if (x64 && sizeof(T) != 4) return cudaErrorInvalidValue;
+    if (!wls && !apic) return launch_g2p_kind<D, T, BW, G_PLAIN>(M, G, P, s, b, cfg, count_next, x64, vm);
+    if (!apic) return launch_g2p_kind<D, T, BW, G_WLS>(M, G, P, s, b, cfg, count_next, x64, vm);
+    if (wls) return launch_g2p_kind<D, T, BW, G_WLS_APIC>(M, G, P, s, b, cfg, count_next, x64, vm);
+    return launch_g2p_kind<D, T, BW, G_APIC>(M, G, P, s, b, cfg, count_next, x64, vm);
 }
 
 template <int D, class T>
