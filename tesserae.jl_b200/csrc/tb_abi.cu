@@ -982,7 +982,7 @@ int check_adjoint_params(tb_ctx* c, const tb_step_params* p) {
 
 // The separable, block-scheduled adjoint kernels cover the quadratic B-spline
 // and uGIMP with FLIP/PIC; every other basis and APIC take the general
-// (particle-parallel, Dual3) reverse step.
+// (particle-parallel, Dual1) reverse step.
 bool adjoint_is_general(const tb_step_params* p) {
     return !(p->basis == TB_BSPLINE_QUADRATIC || p->basis == TB_UGIMP) || p->transfer == TB_TRANSFER_APIC;
 }

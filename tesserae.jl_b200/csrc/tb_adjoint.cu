@@ -896,137 +896,177 @@ __global__ void __launch_bounds__(256) adj_material_kernel(PView<T> P, Scalars<T
 
 // ---------------------------------------------------------------------------
 // General reverse step (WLS and KernelCorrection bases, the APIC transfer): the
-// oracle's general reverse step on the device, one thread per particle. The
-// weights N_i, grad N_i and their derivatives with respect to x_p come from the
-// basis evaluated in Dual3 (value plus the three x_p derivatives), so no
-// second derivative of a WLS or corrected kernel is written out by hand. The
-// v / vn sensitivities of G2P backwards are scattered with FP64 global atomics
-// (27 nodes x 2D per particle); P2G backwards gathers m_bar, mv_bar, f_bar over
-// the window and leaves sigma_bar, V_bar for adj_material_kernel.
-// The mesh in Dual3: the state type's spacing and origin, or the FP64 ones in
+// oracle's general reverse step on the device, one thread per particle. Every
+// weight of this path is built per axis (N_i = W_i - u . G_i with product jets W, G;
+// KernelCorrection corrects the axis jets), and an axis's jets depend on that axis's
+// coordinate only: the basis is evaluated once per particle in Dual1 (value and
+// derivative with respect to the own coordinate), which gives per axis slot
+// (a, a', g, g') and per axis (u, u'), and the derivatives of N and grad N at a node are
+// products of those. The sums over the window are taken row by row (x first), so a
+// node costs about 50 multiply-adds. The y and z jets of a thread live in shared
+// memory, where the row loops may index them; the x jets in registers.
+// The v / vn sensitivities of G2P backwards are scattered with FP64 global atomics
+// (27 nodes x D with APIC, x 2D with FLIP); P2G backwards gathers m_bar, mv_bar, f_bar
+// over the window and leaves sigma_bar, V_bar for adj_material_kernel.
+// 281 k particles, WLS(uGIMP) + APIC: 0.77 + 0.80 ms per step with the weights and a
+// moment inverse in three-derivative duals at every node (0.34 + 0.45 ms with the
+// closed-form weights), 0.14 + 0.25 ms here.
+
+// The mesh in Dual1: the state type's spacing and origin, or the FP64 ones in
 // the FP64-position form (whose forward windows come from them).
 template <int D, class T>
-__device__ __forceinline__ DMesh<D, Dual3> dual_mesh(const DMesh<D, T>& M, bool x64) {
-    DMesh<D, Dual3> R;
+__device__ __forceinline__ DMesh<D, Dual1> dual_mesh(const DMesh<D, T>& M, bool x64) {
+    DMesh<D, Dual1> R;
     for (int d = 0; d < 3; ++d) {
         R.n[d] = M.n[d];
         R.nb[d] = M.nb[d];
-        R.xmin[d] = Dual3(x64 ? M.xmin64[d] : double(M.xmin[d]));
+        R.xmin[d] = Dual1(x64 ? M.xmin64[d] : double(M.xmin[d]));
         R.xmin64[d] = M.xmin64[d];
     }
     R.L = M.L;
     R.nblocks = M.nblocks;
     R.nnodes = M.nnodes;
-    R.h = Dual3(x64 ? M.h64 : double(M.h));
-    R.h_inv = Dual3(x64 ? M.h_inv64 : double(M.h_inv));
+    R.h = Dual1(x64 ? M.h64 : double(M.h));
+    R.h_inv = Dual1(x64 ? M.h_inv64 : double(M.h_inv));
     R.h64 = M.h64;
     R.h_inv64 = M.h_inv64;
     return R;
 }
 
-// Basis of particle x in Dual3: dual seeds e_0 .. e_{D-1} on the position.
-template <int D, class T>
-__device__ __forceinline__ bool dual_basis(const DMesh<D, Dual3>& MD, const Scalars<T>& s, const double* x, T l,
-                                           Basis<D, Dual3>& B, int* err) {
-    Dual3 xd[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        xd[d] = Dual3(d < D ? x[d] : 0.0);
-        if (d < D) xd[d].d[d] = 1.0;
-    }
-    GimpLen<Dual3> gl;
-    gl.ln64 = double(l) / MD.h.v;
-    gl.ln = Dual3(gl.ln64);
-    gl.il = Dual3(1.0 / gl.ln64);
-    return prepare_basis<D, Dual3, true>(MD, s.basis, xd, gl, B, err);
-}
+constexpr int GEN_ADJ_THREADS = 128;
 
-// N, grad N (values and x_p derivatives) at window slot (i, j, k).
+// One axis slot: W's factor and its derivative, grad W's factor and its derivative.
+struct AxisJet {
+    double a, a1, g, g1;
+};
+
+// The jets of one particle: x slots in registers, y and z slots in shared memory
+// (`sh`, [12 (D - 1)][GEN_ADJ_THREADS], this thread's column), u and u' (WLS).
 template <int D>
-__device__ __forceinline__ void dual_node(const DMesh<D, Dual3>& MD, const Basis<D, Dual3>& B, int i, int j, int k,
-                                          Dual3& N, Dual3* G) {
-    eval_node<D, Dual3>(MD, B, i, j, k, N, G);
-}
+struct GenJets {
+    int lo[3], cnt[3];
+    AxisJet x[3];
+    double u[3], u1[3], r0[3];  // r0: X_lo - x_p
+    double* sh;
+    __device__ __forceinline__ AxisJet at(int d, int k) const {  // d = 1, 2
+        const double* q = sh + 4 * (3 * (d - 1) + k) * GEN_ADJ_THREADS;
+        return {q[0], q[GEN_ADJ_THREADS], q[2 * GEN_ADJ_THREADS], q[3 * GEN_ADJ_THREADS]};
+    }
+    template <class T>
+    __device__ __forceinline__ bool prepare(const DMesh<D, T>& M, const Scalars<T>& s, const double* x, bool x64, T l,
+                                            int* err) {
+        const DMesh<D, Dual1> MD = dual_mesh<D, T>(M, x64);
+        Dual1 xd[3];
+#pragma unroll
+        for (int d = 0; d < D; ++d) {  // each axis's jets see their own coordinate only
+            xd[d] = Dual1(x[d]);
+            xd[d].d = 1.0;
+        }
+        GimpLen<Dual1> gl;
+        gl.ln64 = double(l) / MD.h.v;
+        gl.ln = Dual1(gl.ln64);
+        gl.il = Dual1(1.0 / gl.ln64);
+        Basis<D, Dual1> B;
+        if (!prepare_basis<D, Dual1, true>(MD, s.basis, xd, gl, B, err)) return false;
+        const double hi = MD.h_inv.v;
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+            lo[d] = B.ax[d].lo;
+            cnt[d] = B.ax[d].cnt;
+            u[d] = B.wls ? B.u[d].v : 0.0;
+            u1[d] = B.wls ? B.u[d].d : 0.0;
+            r0[d] = __dadd_rn(M.xmin64[d], __dmul_rn(double(lo[d]), M.h64)) - x[d];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const AxisJet q = {B.ax[d].val[k].v, B.ax[d].val[k].d, B.ax[d].der[k].v * hi, B.ax[d].der[k].d * hi};
+                if (d == 0) {
+                    x_slot(k) = q;
+                } else {
+                    double* w = sh + 4 * (3 * (d - 1) + k) * GEN_ADJ_THREADS;
+                    w[0] = q.a;
+                    w[GEN_ADJ_THREADS] = q.a1;
+                    w[2 * GEN_ADJ_THREADS] = q.g;
+                    w[3 * GEN_ADJ_THREADS] = q.g1;
+                }
+            }
+        }
+        return true;
+    }
+    __device__ __forceinline__ AxisJet& x_slot(int k) { return x[k]; }
+};
+
+// The factors of a window row (y, z fixed): with the x jets (a, a', g, g')
+//   N = a R + g Q, dN/dx = a' R + g' Q + g Q', dN/dy = a Ry + g Qy, dN/dz = a Rz + g Qz
+//   G_x = g yz, G_y = a gyz, G_z = a ygz,
+//   dG_x = (g' yz, g y1z, g yz1), dG_y = (a' gyz, a g1yz, a gyz1), dG_z = (a' ygz, a y1gz, a ygz1).
+template <int D>
+struct RowFactors {
+    double yz, y1z, yz1, gyz, g1yz, gyz1, ygz, y1gz, ygz1;
+    double R, Ry, Rz, Q, Qx, Qy, Qz;
+    __device__ __forceinline__ RowFactors(const GenJets<D>& J, int j, int k) {
+        const AxisJet y = J.at(1, j);
+        AxisJet z = {1.0, 0.0, 0.0, 0.0};
+        if constexpr (D == 3) z = J.at(2, k);
+        yz = y.a * z.a;
+        y1z = y.a1 * z.a;
+        yz1 = y.a * z.a1;
+        gyz = y.g * z.a;
+        g1yz = y.g1 * z.a;
+        gyz1 = y.g * z.a1;
+        ygz = y.a * z.g;
+        y1gz = y.a1 * z.g;
+        ygz1 = y.a * z.g1;
+        const double u2 = D == 3 ? J.u[D - 1] : 0.0, u21 = D == 3 ? J.u1[D - 1] : 0.0;
+        R = yz - J.u[1] * gyz - u2 * ygz;
+        Ry = y1z - J.u[1] * g1yz - J.u1[1] * gyz - u2 * y1gz;
+        Rz = yz1 - J.u[1] * gyz1 - u2 * ygz1 - u21 * ygz;
+        Q = -J.u[0] * yz;
+        Qx = -J.u1[0] * yz;
+        Qy = -J.u[0] * y1z;
+        Qz = -J.u[0] * yz1;
+    }
+};
 
 template <int D, class T>
-__global__ void __launch_bounds__(128) adj_g2p_gen_kernel(DMesh<D, T> M, GView<T> G, PView<T> P, Scalars<T> s,
-                                                          AdjView A, GradGrid GB, const int* __restrict__ blockids,
-                                                          int* err) {
-    const DMesh<D, Dual3> MD = dual_mesh<D, T>(M, P.x64[0] != nullptr);
-    const bool apic = s.transfer == TB_TRANSFER_APIC;
+__global__ void __launch_bounds__(GEN_ADJ_THREADS) adj_g2p_gen_kernel(DMesh<D, T> M, GView<T> G, PView<T> P,
+                                                                      Scalars<T> s, AdjView A, GradGrid GB,
+                                                                      const int* __restrict__ blockids, int* err) {
+    __shared__ double sh[12 * (D - 1) * GEN_ADJ_THREADS];
+    const bool apic = s.transfer == TB_TRANSFER_APIC, x64 = P.x64[0] != nullptr;
     const double dt = s.dt64, alpha = double(s.alpha);
     for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < P.n;
          p += (long long)gridDim.x * blockDim.x) {
         double x[3];
         load_xd<D, T>(P, p, x);
-        const T l = P.l ? P.l[p] : s.gimp_l;
-        Basis<D, Dual3> B;
-        const bool in = blockids[p] != 0 && dual_basis<D, T>(MD, s, x, l, B, err);
-        double F[3][3] = {}, Fb[3][3] = {}, L[3][3] = {};
-        load_F<D, T>(P, p, F);
+        GenJets<D> J;
+        J.sh = sh + threadIdx.x;
+        const bool in = blockids[p] != 0 && J.prepare(M, s, x, x64, P.l ? P.l[p] : s.gimp_l, err);
+        double Lb[3][3] = {};  // dt F_bar F^T
+        {
+            double F[3][3] = {}, Fb[3][3] = {};
+            load_F<D, T>(P, p, F);
 #pragma unroll
-        for (int r = 0; r < D; ++r)
+            for (int r = 0; r < D; ++r)
 #pragma unroll
-            for (int c = 0; c < D; ++c) Fb[r][c] = A.F[r + c * D][p];
-        auto node_of = [&](int i, int j, int k, long long& I, Dual3 (&rel)[3], bool& valid) {
-            const int idx[3] = {i, j, k};
-            I = 0;
-            valid = true;
+                for (int c = 0; c < D; ++c) Fb[r][c] = A.F[r + c * D][p];
 #pragma unroll
-            for (int d = D - 1; d >= 0; --d) {
-                valid = valid && idx[d] < B.ax[d].cnt;
-                I = I * M.n[d] + min(B.ax[d].lo + idx[d], M.n[d] - 1);
-            }
+            for (int r = 0; r < D; ++r)
 #pragma unroll
-            for (int d = 0; d < 3; ++d) rel[d] = Dual3(0.0);
+                for (int c = 0; c < D; ++c) {
+                    double s2 = 0.0;
 #pragma unroll
-            for (int d = 0; d < D; ++d) {
-                rel[d] = node_coord(MD, d, B.ax[d].lo + idx[d]) - Dual3(x[d]);
-                rel[d].d[d] = -1.0;
-            }
-        };
-        if (in) {
-            for (int k = 0; k < (D == 3 ? 3 : 1); ++k)
-                for (int j = 0; j < 3; ++j)
-                    for (int i = 0; i < 3; ++i) {
-                        long long I;
-                        Dual3 rel[3];
-                        bool valid;
-                        node_of(i, j, k, I, rel, valid);
-                        if (!valid) continue;
-                        Dual3 N, Gn[3];
-                        dual_node<D>(MD, B, i, j, k, N, Gn);
-#pragma unroll
-                        for (int r = 0; r < D; ++r)
-#pragma unroll
-                            for (int c = 0; c < D; ++c) L[r][c] += double(G.v[r][I]) * Gn[c].v;
-                    }
-        }
-        double Lb[3][3] = {}, Fbn[3][3] = {};
-#pragma unroll
-        for (int r = 0; r < D; ++r)
-#pragma unroll
-            for (int c = 0; c < D; ++c) {
-                double s1 = 0.0, s2 = 0.0;
-#pragma unroll
-                for (int q = 0; q < D; ++q) {
-                    s1 += ((r == q ? 1.0 : 0.0) + dt * L[q][r]) * Fb[q][c];
-                    s2 += Fb[r][q] * F[c][q];
+                    for (int q = 0; q < D; ++q) s2 += Fb[r][q] * F[c][q];
+                    Lb[r][c] = dt * s2;
                 }
-                Fbn[r][c] = s1;
-                Lb[r][c] = dt * s2;
-            }
-        double xb[3] = {}, vbp[3] = {}, vpicb[3] = {}, dvb[3] = {}, Bb[3][3] = {};
+        }
+        double xb[3] = {}, vpicb[3] = {}, dvb[3] = {}, Bb[3][3] = {}, L[3][3] = {};
 #pragma unroll
         for (int d = 0; d < D; ++d) {
             xb[d] = A.x[d][p];
-            vbp[d] = A.v[d][p];
-            if (apic) {
-                vpicb[d] = vbp[d] + dt * xb[d];
-            } else {
-                dvb[d] = alpha * vbp[d];
-                vpicb[d] = (1.0 - alpha) * vbp[d] + dt * xb[d];
-            }
+            const double vbp = A.v[d][p];
+            dvb[d] = apic ? 0.0 : alpha * vbp;
+            vpicb[d] = (apic ? vbp : (1.0 - alpha) * vbp) + dt * xb[d];
+            A.v[d][p] = apic ? 0.0 : alpha * vbp;
         }
         if (apic) {
 #pragma unroll
@@ -1035,74 +1075,103 @@ __global__ void __launch_bounds__(128) adj_g2p_gen_kernel(DMesh<D, T> M, GView<T
                 for (int c = 0; c < D; ++c) Bb[r][c] = A.B[r + c * D][p];
         }
         if (in) {
-            for (int k = 0; k < (D == 3 ? 3 : 1); ++k)
-                for (int j = 0; j < 3; ++j)
-                    for (int i = 0; i < 3; ++i) {
-                        long long I;
-                        Dual3 rel[3];
-                        bool valid;
-                        node_of(i, j, k, I, rel, valid);
-                        if (!valid) continue;
-                        Dual3 N, Gn[3];
-                        dual_node<D>(MD, B, i, j, k, N, Gn);
-                        double vi[3] = {}, vni[3] = {};
+#pragma unroll 1
+            for (int k = 0; k < (D == 3 ? min(3, J.cnt[D - 1]) : 1); ++k)
+#pragma unroll 1
+                for (int j = 0; j < J.cnt[1]; ++j) {
+                    const RowFactors<D> f(J, j, k);
+                    const long long I0 = (long long)J.lo[0] +
+                                         (long long)M.n[0] * ((J.lo[1] + j) + (D == 3 ? (long long)M.n[1] * (J.lo[D - 1] + k) : 0ll));
+                    // the row's part of the APIC affine term and of Lb G
+                    const double ry = J.r0[1] + double(j) * M.h64, rz = D == 3 ? J.r0[D - 1] + double(k) * M.h64 : 0.0;
+                    double cr[3] = {}, La[3] = {};
 #pragma unroll
-                        for (int d = 0; d < D; ++d) {
-                            vi[d] = double(G.v[d][I]);
-                            vni[d] = double(G.vn[d][I]);
-                        }
-                        double Nb = 0.0, Gb[3] = {0.0, 0.0, 0.0};
+                    for (int r = 0; r < D; ++r) {
+                        cr[r] = vpicb[r];
+                        if (apic) cr[r] += Bb[r][1] * ry + (D == 3 ? Bb[r][D - 1] * rz : 0.0);
+                        La[r] = Lb[r][1] * f.gyz + (D == 3 ? Lb[r][D - 1] * f.ygz : 0.0);
+                    }
+                    double av[3] = {}, gv[3] = {};                       // sum a v, sum g v
+                    double na = 0.0, na1 = 0.0, ng = 0.0, ng1 = 0.0;      // of Nb
+                    double t0g = 0.0, t0g1 = 0.0, t1a = 0.0, t1a1 = 0.0, t2a = 0.0, t2a1 = 0.0;  // of Gb
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) {
+                        if (i >= J.cnt[0]) continue;
+                        const AxisJet q = J.x[i];
+                        const long long I = I0 + i;
+                        const double N = q.a * f.R + q.g * f.Q, gx = q.g * f.yz;
+                        const double rx = J.r0[0] + double(i) * M.h64;
+                        double Nb = 0.0, Gb[3] = {};
 #pragma unroll
                         for (int r = 0; r < D; ++r) {
-                            double vb_r = N.v * (vpicb[r] + dvb[r]);
+                            const double vi = double(G.v[r][I]);
+                            double c = cr[r];
+                            if (apic) c += Bb[r][0] * rx;
+                            Nb += c * vi;
+                            if (!apic) Nb += dvb[r] * (vi - double(G.vn[r][I]));
 #pragma unroll
-                            for (int c = 0; c < D; ++c) vb_r += Lb[r][c] * Gn[c].v;
-                            Nb += vpicb[r] * vi[r] + dvb[r] * (vi[r] - vni[r]);
-#pragma unroll
-                            for (int c = 0; c < D; ++c) Gb[c] += Lb[r][c] * vi[r];
-                            if (apic) {
-                                double Br = 0.0;
-#pragma unroll
-                                for (int c = 0; c < D; ++c) {
-                                    Br += Bb[r][c] * rel[c].v;
-                                    xb[c] -= N.v * vi[r] * Bb[r][c];
-                                }
-                                vb_r += N.v * Br;
-                                Nb += vi[r] * Br;
-                            }
-                            atomicAdd(GB.vb[r] + I, vb_r);
-                            if (!apic) atomicAdd(GB.vnb[r] + I, -N.v * dvb[r]);
+                            for (int d = 0; d < D; ++d) Gb[d] += Lb[r][d] * vi;
+                            av[r] += q.a * vi;
+                            gv[r] += q.g * vi;
+                            atomicAdd(GB.vb[r] + I, N * (c + dvb[r]) + gx * Lb[r][0] + q.a * La[r]);
+                            if (!apic) atomicAdd(GB.vnb[r] + I, -N * dvb[r]);
                         }
-#pragma unroll
-                        for (int b = 0; b < D; ++b) {
-                            double h = 0.0;
-#pragma unroll
-                            for (int c = 0; c < D; ++c) h += Gb[c] * Gn[c].d[b];
-                            xb[b] += Nb * N.d[b] + h;
+                        na += q.a * Nb;
+                        na1 += q.a1 * Nb;
+                        ng += q.g * Nb;
+                        ng1 += q.g1 * Nb;
+                        t0g += q.g * Gb[0];
+                        t0g1 += q.g1 * Gb[0];
+                        t1a += q.a * Gb[1];
+                        t1a1 += q.a1 * Gb[1];
+                        if constexpr (D == 3) {
+                            t2a += q.a * Gb[D - 1];
+                            t2a1 += q.a1 * Gb[D - 1];
                         }
                     }
+#pragma unroll
+                    for (int r = 0; r < D; ++r) {
+                        L[r][0] += f.yz * gv[r];
+                        L[r][1] += f.gyz * av[r];
+                        if constexpr (D == 3) L[r][D - 1] += f.ygz * av[r];
+                        if (apic) {
+                            const double Nv = f.R * av[r] + f.Q * gv[r];
+#pragma unroll
+                            for (int c = 0; c < D; ++c) xb[c] -= Nv * Bb[r][c];
+                        }
+                    }
+                    xb[0] += na1 * f.R + ng1 * f.Q + ng * f.Qx + t0g1 * f.yz + t1a1 * f.gyz + t2a1 * f.ygz;
+                    xb[1] += na * f.Ry + ng * f.Qy + t0g * f.y1z + t1a * f.g1yz + t2a * f.y1gz;
+                    if constexpr (D == 3) xb[D - 1] += na * f.Rz + ng * f.Qz + t0g * f.yz1 + t1a * f.gyz1 + t2a * f.ygz1;
+                }
         }
 #pragma unroll
-        for (int d = 0; d < D; ++d) {
-            A.x[d][p] = xb[d];
-            A.v[d][p] = apic ? 0.0 : alpha * vbp[d];
-        }
+        for (int d = 0; d < D; ++d) A.x[d][p] = xb[d];
+        double Fb[3][3] = {};
+#pragma unroll
+        for (int r = 0; r < D; ++r)
+#pragma unroll
+            for (int c = 0; c < D; ++c) Fb[r][c] = A.F[r + c * D][p];
 #pragma unroll
         for (int r = 0; r < D; ++r)
 #pragma unroll
             for (int c = 0; c < D; ++c) {
-                A.F[r + c * D][p] = Fbn[r][c];
+                double s1 = 0.0;
+#pragma unroll
+                for (int q = 0; q < D; ++q) s1 += ((r == q ? 1.0 : 0.0) + dt * L[q][r]) * Fb[q][c];
+                A.F[r + c * D][p] = s1;
                 if (apic) A.B[r + c * D][p] = 0.0;
             }
     }
 }
 
 template <int D, class T>
-__global__ void __launch_bounds__(128) adj_p2g_gen_kernel(DMesh<D, T> M, PView<T> P, Scalars<T> s, AdjView A,
-                                                          GradGrid GB, double* __restrict__ sbar,
-                                                          const int* __restrict__ blockids, int* err) {
-    const DMesh<D, Dual3> MD = dual_mesh<D, T>(M, P.x64[0] != nullptr);
-    const bool apic = s.transfer == TB_TRANSFER_APIC;
+__global__ void __launch_bounds__(GEN_ADJ_THREADS) adj_p2g_gen_kernel(DMesh<D, T> M, PView<T> P, Scalars<T> s,
+                                                                      AdjView A, GradGrid GB,
+                                                                      double* __restrict__ sbar,
+                                                                      const int* __restrict__ blockids, int* err) {
+    __shared__ double sh[12 * (D - 1) * GEN_ADJ_THREADS];
+    const bool apic = s.transfer == TB_TRANSFER_APIC, x64 = P.x64[0] != nullptr;
     const double dinv = 4.0 / (double(M.h) * double(M.h));
     const long long n = P.n;
     for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < n;
@@ -1110,101 +1179,116 @@ __global__ void __launch_bounds__(128) adj_p2g_gen_kernel(DMesh<D, T> M, PView<T
         if (blockids[p] == 0) continue;
         double x[3];
         load_xd<D, T>(P, p, x);
-        const T l = P.l ? P.l[p] : s.gimp_l;
-        Basis<D, Dual3> B;
-        if (!dual_basis<D, T>(MD, s, x, l, B, err)) continue;
+        GenJets<D> J;
+        J.sh = sh + threadIdx.x;
+        if (!J.prepare(M, s, x, x64, P.l ? P.l[p] : s.gimp_l, err)) continue;
         const double mp = P.m ? double(P.m[p]) : double(s.mass);
         const double Vp = double(P.V[p]);
-        double vp[3] = {}, Bp[3][3] = {}, sg[3][3] = {};
+        // m v_p and m D^-1 B_p, -V sigma
+        double mv[3] = {}, mB[3][3] = {}, S[3][3] = {};
 #pragma unroll
-        for (int d = 0; d < D; ++d) vp[d] = double(P.v[d][p]);
+        for (int d = 0; d < D; ++d) mv[d] = mp * double(P.v[d][p]);
 #pragma unroll
         for (int r = 0; r < D; ++r)
 #pragma unroll
             for (int c = 0; c < D; ++c) {
-                sg[r][c] = double(P.sig[symidx<D>(r, c)][p]);
-                if (apic) Bp[r][c] = double(P.B[r + c * D][p]);
+                S[r][c] = -Vp * double(P.sig[symidx<D>(r, c)][p]);
+                if (apic) mB[r][c] = mp * dinv * double(P.B[r + c * D][p]);
             }
-        double xb[3] = {}, vbs[3] = {}, sb[3][3] = {}, Vb = 0.0, Bbs[3][3] = {};
-        for (int k = 0; k < (D == 3 ? 3 : 1); ++k)
-            for (int j = 0; j < 3; ++j)
+        // xb, sum N p_bar, sum N p_bar r, sum f_bar (x) G
+        double xb[3] = {}, np[3] = {}, npr[3][3] = {}, fG[3][3] = {};
+#pragma unroll 1
+        for (int k = 0; k < (D == 3 ? min(3, J.cnt[D - 1]) : 1); ++k)
+#pragma unroll 1
+            for (int j = 0; j < J.cnt[1]; ++j) {
+                const RowFactors<D> f(J, j, k);
+                const long long I0 = (long long)J.lo[0] +
+                                     (long long)M.n[0] * ((J.lo[1] + j) + (D == 3 ? (long long)M.n[1] * (J.lo[D - 1] + k) : 0ll));
+                const double ry = J.r0[1] + double(j) * M.h64, rz = D == 3 ? J.r0[D - 1] + double(k) * M.h64 : 0.0;
+                double U[3] = {};
+#pragma unroll
+                for (int d = 0; d < D; ++d) {
+                    U[d] = mv[d];
+                    if (apic) U[d] += mB[d][1] * ry + (D == 3 ? mB[d][D - 1] * rz : 0.0);
+                }
+                double pa[3] = {}, pg[3] = {}, par[3] = {}, pgr[3] = {}, fa[3] = {}, fg[3] = {};
+                double na = 0.0, na1 = 0.0, ng = 0.0, ng1 = 0.0;
+                double t0g = 0.0, t0g1 = 0.0, t1a = 0.0, t1a1 = 0.0, t2a = 0.0, t2a1 = 0.0;
+#pragma unroll
                 for (int i = 0; i < 3; ++i) {
-                    const int idx[3] = {i, j, k};
-                    long long I = 0;
-                    bool valid = true;
-#pragma unroll
-                    for (int d = D - 1; d >= 0; --d) {
-                        valid = valid && idx[d] < B.ax[d].cnt;
-                        I = I * M.n[d] + min(B.ax[d].lo + idx[d], M.n[d] - 1);
-                    }
-                    if (!valid) continue;
-                    Dual3 rel[3];
-#pragma unroll
-                    for (int d = 0; d < 3; ++d) rel[d] = Dual3(0.0);
-#pragma unroll
-                    for (int d = 0; d < D; ++d) {
-                        rel[d] = node_coord(MD, d, B.ax[d].lo + idx[d]) - Dual3(x[d]);
-                        rel[d].d[d] = -1.0;
-                    }
-                    Dual3 N, Gn[3];
-                    dual_node<D>(MD, B, i, j, k, N, Gn);
-                    double u[3] = {};
-#pragma unroll
-                    for (int d = 0; d < D; ++d) {
-                        u[d] = vp[d];
-                        if (apic)
-#pragma unroll
-                            for (int c = 0; c < D; ++c) u[d] += Bp[d][c] * dinv * rel[c].v;
-                    }
-                    double Nb = mp * GB.mb[I], Gb[3] = {0.0, 0.0, 0.0};
+                    if (i >= J.cnt[0]) continue;
+                    const AxisJet q = J.x[i];
+                    const long long I = I0 + i;
+                    const double rx = J.r0[0] + double(i) * M.h64;
+                    double Nb = mp * GB.mb[I], t[3] = {};
 #pragma unroll
                     for (int d = 0; d < D; ++d) {
                         const double p_b = GB.pb[d][I], f_b = GB.fb[d][I];
-                        Nb += mp * (u[d] * p_b + double(s.g[d]) * f_b);
-                        const double ub = mp * N.v * p_b;
-                        vbs[d] += ub;
-                        if (apic)
-#pragma unroll
-                            for (int c = 0; c < D; ++c) {
-                                Bbs[d][c] += ub * dinv * rel[c].v;
-                                xb[c] -= ub * Bp[d][c] * dinv;
-                            }
-                    }
-#pragma unroll
-                    for (int r = 0; r < D; ++r) {
-                        const double f_b = GB.fb[r][I];
-                        double sgg = 0.0;
-#pragma unroll
-                        for (int c = 0; c < D; ++c) {
-                            sgg += sg[r][c] * Gn[c].v;
-                            Gb[c] += -Vp * sg[r][c] * f_b;
-                            sb[r][c] += -Vp * f_b * Gn[c].v;
+                        double ud = U[d];
+                        if (apic) ud += mB[d][0] * rx;
+                        Nb += ud * p_b + (mp * double(s.g[d])) * f_b;
+                        pa[d] += q.a * p_b;
+                        pg[d] += q.g * p_b;
+                        if (apic) {
+                            par[d] += (q.a * rx) * p_b;
+                            pgr[d] += (q.g * rx) * p_b;
                         }
-                        Vb += -f_b * sgg;
+                        fa[d] += q.a * f_b;
+                        fg[d] += q.g * f_b;
+#pragma unroll
+                        for (int c = 0; c < D; ++c) t[c] += S[d][c] * f_b;
                     }
-#pragma unroll
-                    for (int b = 0; b < D; ++b) {
-                        double h = 0.0;
-#pragma unroll
-                        for (int c = 0; c < D; ++c) h += Gb[c] * Gn[c].d[b];
-                        xb[b] += Nb * N.d[b] + h;
+                    na += q.a * Nb;
+                    na1 += q.a1 * Nb;
+                    ng += q.g * Nb;
+                    ng1 += q.g1 * Nb;
+                    t0g += q.g * t[0];
+                    t0g1 += q.g1 * t[0];
+                    t1a += q.a * t[1];
+                    t1a1 += q.a1 * t[1];
+                    if constexpr (D == 3) {
+                        t2a += q.a * t[D - 1];
+                        t2a1 += q.a1 * t[D - 1];
                     }
                 }
 #pragma unroll
+                for (int d = 0; d < D; ++d) {
+                    const double Np = f.R * pa[d] + f.Q * pg[d];
+                    np[d] += Np;
+                    if (apic) {
+                        npr[d][0] += f.R * par[d] + f.Q * pgr[d];
+                        npr[d][1] += Np * ry;
+                        if constexpr (D == 3) npr[d][D - 1] += Np * rz;
+                    }
+                    fG[d][0] += f.yz * fg[d];
+                    fG[d][1] += f.gyz * fa[d];
+                    if constexpr (D == 3) fG[d][D - 1] += f.ygz * fa[d];
+                }
+                xb[0] += na1 * f.R + ng1 * f.Q + ng * f.Qx + t0g1 * f.yz + t1a1 * f.gyz + t2a1 * f.ygz;
+                xb[1] += na * f.Ry + ng * f.Qy + t0g * f.y1z + t1a * f.g1yz + t2a * f.y1gz;
+                if constexpr (D == 3) xb[D - 1] += na * f.Rz + ng * f.Qz + t0g * f.yz1 + t1a * f.gyz1 + t2a * f.ygz1;
+            }
+        double Vb = 0.0;
+#pragma unroll
         for (int d = 0; d < D; ++d) {
-            A.x[d][p] += xb[d];
-            A.v[d][p] += vbs[d];
-        }
-        if (apic) {
+            if (apic) {
 #pragma unroll
-            for (int r = 0; r < D; ++r)
-#pragma unroll
-                for (int c = 0; c < D; ++c) A.B[r + c * D][p] += Bbs[r][c];
+                for (int c = 0; c < D; ++c) {
+                    xb[c] -= np[d] * mB[d][c];
+                    A.B[d + c * D][p] += mp * dinv * npr[d][c];
+                }
+            }
+            A.v[d][p] += mp * np[d];
         }
+#pragma unroll
+        for (int d = 0; d < D; ++d) A.x[d][p] += xb[d];
 #pragma unroll
         for (int r = 0; r < D; ++r)
 #pragma unroll
-            for (int c = 0; c < D; ++c) sbar[(r * D + c) * n + p] = sb[r][c];
+            for (int c = 0; c < D; ++c) {
+                sbar[(r * D + c) * n + p] = -Vp * fG[r][c];
+                Vb -= double(P.sig[symidx<D>(r, c)][p]) * fG[r][c];
+            }
         sbar[D * D * n + p] = Vb;
     }
 }
@@ -1294,7 +1378,7 @@ cudaError_t launch_adjoint_general(const DMesh<D, T>& M, const GView<T>& G, cons
     const int ngrid = int(std::max<long long>(1, std::min<long long>((M.nnodes + 255) / 256, (long long)cfg.num_sms * 8)));
     if (P.n > 0) {
         KernelScope ks(cfg, "adj_g2p");
-        adj_g2p_gen_kernel<D, T><<<pgrid, 128, 0, cfg.stream>>>(M, G, P, s, A, GB, part.blockids, cfg.err);
+        adj_g2p_gen_kernel<D, T><<<pgrid, GEN_ADJ_THREADS, 0, cfg.stream>>>(M, G, P, s, A, GB, part.blockids, cfg.err);
         ++*cfg.launches;
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
@@ -1307,7 +1391,7 @@ cudaError_t launch_adjoint_general(const DMesh<D, T>& M, const GView<T>& G, cons
     if (P.n > 0) {
         {
             KernelScope ks(cfg, "adj_p2g");
-            adj_p2g_gen_kernel<D, T><<<pgrid, 128, 0, cfg.stream>>>(M, P, s, A, GB, GB.coef, part.blockids, cfg.err);
+            adj_p2g_gen_kernel<D, T><<<pgrid, GEN_ADJ_THREADS, 0, cfg.stream>>>(M, P, s, A, GB, GB.coef, part.blockids, cfg.err);
             ++*cfg.launches;
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
         }

@@ -80,65 +80,66 @@ struct BlockPasses {
     __device__ __forceinline__ int step(int nt) const { return npass * nt; }
 };
 
-// Forward-mode dual number with the three derivatives with respect to a
-// particle's position: the weights evaluated in Dual3 give dN/dx_p and
-// d(grad N)/dx_p for the reverse step of every basis (WLS, KernelCorrection,
-// truncated windows) without hand-derived second derivatives. Floors and
+// Forward-mode dual number: a value and its derivative with respect to one
+// coordinate of the particle. Every basis of this path is built axis by axis, so
+// one derivative (of each axis's jets with respect to that axis's coordinate) gives
+// dN/dx_p and d(grad N)/dx_p of the reverse step for every basis (WLS,
+// KernelCorrection, cut windows) without hand-derived second derivatives. Floors and
 // comparisons act on the value, |x| follows the value's sign. In a namespace of
 // its own, so that floor, fabs and signbit of plain numbers inside tb still
-// resolve to the CUDA functions (the Dual3 overloads are found by argument-
+// resolve to the CUDA functions (the Dual1 overloads are found by argument-
 // dependent lookup).
 namespace ad {
-struct Dual3 {
-    double v, d[3];
-    __host__ __device__ Dual3() : v(0.0), d{0.0, 0.0, 0.0} {}
-    __host__ __device__ Dual3(double a) : v(a), d{0.0, 0.0, 0.0} {}
+struct Dual1 {
+    double v, d;
+    __host__ __device__ Dual1() : v(0.0), d(0.0) {}
+    __host__ __device__ Dual1(double a) : v(a), d(0.0) {}
     __host__ __device__ explicit operator double() const { return v; }
     __host__ __device__ explicit operator float() const { return float(v); }
     __host__ __device__ explicit operator int() const { return int(v); }
-    __host__ __device__ Dual3 operator-() const {
-        Dual3 r;
+    __host__ __device__ Dual1 operator-() const {
+        Dual1 r;
         r.v = -v;
-        for (int k = 0; k < 3; ++k) r.d[k] = -d[k];
+        r.d = -d;
         return r;
     }
-    __host__ __device__ Dual3& operator+=(const Dual3& o) {
+    __host__ __device__ Dual1& operator+=(const Dual1& o) {
         v += o.v;
-        for (int k = 0; k < 3; ++k) d[k] += o.d[k];
+        d += o.d;
         return *this;
     }
-    __host__ __device__ Dual3& operator-=(const Dual3& o) {
+    __host__ __device__ Dual1& operator-=(const Dual1& o) {
         v -= o.v;
-        for (int k = 0; k < 3; ++k) d[k] -= o.d[k];
+        d -= o.d;
         return *this;
     }
-    __host__ __device__ Dual3& operator*=(const Dual3& o) {
-        for (int k = 0; k < 3; ++k) d[k] = d[k] * o.v + v * o.d[k];
+    __host__ __device__ Dual1& operator*=(const Dual1& o) {
+        d = d * o.v + v * o.d;
         v *= o.v;
         return *this;
     }
-    __host__ __device__ Dual3& operator/=(const Dual3& o) {
+    __host__ __device__ Dual1& operator/=(const Dual1& o) {
         const double iv = 1.0 / o.v;
-        for (int k = 0; k < 3; ++k) d[k] = (d[k] - v * iv * o.d[k]) * iv;
+        d = (d - v * iv * o.d) * iv;
         v *= iv;
         return *this;
     }
 };
-__host__ __device__ inline Dual3 operator+(Dual3 a, const Dual3& b) { return a += b; }
-__host__ __device__ inline Dual3 operator-(Dual3 a, const Dual3& b) { return a -= b; }
-__host__ __device__ inline Dual3 operator*(Dual3 a, const Dual3& b) { return a *= b; }
-__host__ __device__ inline Dual3 operator/(Dual3 a, const Dual3& b) { return a /= b; }
-__host__ __device__ inline bool operator<(const Dual3& a, const Dual3& b) { return a.v < b.v; }
-__host__ __device__ inline bool operator>(const Dual3& a, const Dual3& b) { return a.v > b.v; }
-__host__ __device__ inline bool operator<=(const Dual3& a, const Dual3& b) { return a.v <= b.v; }
-__host__ __device__ inline bool operator>=(const Dual3& a, const Dual3& b) { return a.v >= b.v; }
-__host__ __device__ inline bool operator==(const Dual3& a, const Dual3& b) { return a.v == b.v; }
-__host__ __device__ inline bool operator!=(const Dual3& a, const Dual3& b) { return a.v != b.v; }
-__device__ inline Dual3 floor(const Dual3& a) { return Dual3(::floor(a.v)); }
-__device__ inline Dual3 fabs(const Dual3& a) { return ::signbit(a.v) ? -a : a; }
-__device__ inline bool signbit(const Dual3& a) { return ::signbit(a.v); }
+__host__ __device__ inline Dual1 operator+(Dual1 a, const Dual1& b) { return a += b; }
+__host__ __device__ inline Dual1 operator-(Dual1 a, const Dual1& b) { return a -= b; }
+__host__ __device__ inline Dual1 operator*(Dual1 a, const Dual1& b) { return a *= b; }
+__host__ __device__ inline Dual1 operator/(Dual1 a, const Dual1& b) { return a /= b; }
+__host__ __device__ inline bool operator<(const Dual1& a, const Dual1& b) { return a.v < b.v; }
+__host__ __device__ inline bool operator>(const Dual1& a, const Dual1& b) { return a.v > b.v; }
+__host__ __device__ inline bool operator<=(const Dual1& a, const Dual1& b) { return a.v <= b.v; }
+__host__ __device__ inline bool operator>=(const Dual1& a, const Dual1& b) { return a.v >= b.v; }
+__host__ __device__ inline bool operator==(const Dual1& a, const Dual1& b) { return a.v == b.v; }
+__host__ __device__ inline bool operator!=(const Dual1& a, const Dual1& b) { return a.v != b.v; }
+__device__ inline Dual1 floor(const Dual1& a) { return Dual1(::floor(a.v)); }
+__device__ inline Dual1 fabs(const Dual1& a) { return ::signbit(a.v) ? -a : a; }
+__device__ inline bool signbit(const Dual1& a) { return ::signbit(a.v); }
 }  // namespace ad
-using ad::Dual3;
+using ad::Dual1;
 
 template <int D, class T>
 struct DMesh {
@@ -390,7 +391,7 @@ __device__ __forceinline__ double quotient(double a, double l, double il) {
     const double q = a * il;
     return fma(fma(-q, l, a), il, q);
 }
-__device__ __forceinline__ Dual3 quotient(const Dual3& a, const Dual3& l, const Dual3&) { return a / l; }
+__device__ __forceinline__ Dual1 quotient(const Dual1& a, const Dual1& l, const Dual1&) { return a / l; }
 
 // uGIMP jets (gimp.jl:16-40); il = 1 / l, computed once per particle or per scene.
 // (The nine jets of a 3D particle held 27 divisions by l, about half of the

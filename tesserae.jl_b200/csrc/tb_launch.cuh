@@ -157,7 +157,7 @@ template <int D, class T, int BW>
 cudaError_t launch_adjoint(const DMesh<D, T>& M, const GView<T>& G, const PView<T>& P, const Scalars<T>& s,
                            const AdjView& A, const GradGrid& GB, const AdjPartition& part, const LaunchCfg& cfg);
 // The same for WLS / KernelCorrection bases and the APIC transfer (particle-parallel,
-// weight derivatives in Dual3).
+// weight derivatives in Dual1).
 template <int D, class T>
 cudaError_t launch_adjoint_general(const DMesh<D, T>& M, const GView<T>& G, const PView<T>& P, const Scalars<T>& s,
                                    const AdjView& A, const GradGrid& GB, const AdjPartition& part, const LaunchCfg& cfg);
