@@ -76,7 +76,9 @@ struct tb_ctx {
     long long launches = 0;
     std::string error;
     int* d_err = nullptr;            // device status word (ERR_* bits)
-    int* d_totals = nullptr;         // [2] nactive, nassigned
+    int* d_totals = nullptr;         // [2] nactive, nassigned; then the words below
+    unsigned long long* d_bnd = nullptr;  // [1] blocks of P2G's second launch
+    int* d_touched = nullptr;        // [2] touched-list lengths of even and odd steps
     int* h_totals = nullptr;         // pinned mirror
     // scratch (grow-only)
     int* cursors = nullptr;
@@ -101,8 +103,8 @@ struct tb_ctx {
     long long sp_tot_cap = 0;
     unsigned char* touched_cur = nullptr;
     unsigned char* touched_prev = nullptr;
-    int* touched_list = nullptr;  // [nblocks] blocks with cur or prev set, count in touched_count
-    int* touched_count = nullptr;
+    int* touched_list = nullptr;  // [nblocks] blocks with cur or prev set
+    int touched_parity = 0;       // which of d_touched holds its length
     long long touched_cap = 0;
     const void* grid_key = nullptr;  // grid.m of the grid the flags describe
     long long grid_nblocks = 0;
@@ -323,6 +325,7 @@ int bin_buffers(tb_ctx* c, const tb_partition* part, long long n, long long nb, 
     B.partials = c->partials;
     B.sort_scratch = c->sort_scratch;
     B.totals = c->d_totals;
+    B.bnd_count = c->d_bnd;
     return TB_OK;
 }
 
@@ -390,7 +393,6 @@ int reorder_args(tb_ctx* c, const tb_partition* part, long long n, double thresh
     a.nblocks = int(part->nblocks);
     a.blockids = part->blockids;
     a.perm = part->particleindices;
-    a.counts = part->counts;
     a.offsets = part->offsets;
     a.threshold = threshold;
     a.acc = c->ro_acc;
@@ -410,8 +412,6 @@ int touched_buffers(tb_ctx* c, long long nb) {
         if ((e = grow(c->touched_prev, cap, nb)) != cudaSuccess) return cuda_fail(c, e, "cudaMalloc touched flags");
         cap = c->touched_cap;
         if ((e = grow(c->touched_list, cap, nb)) != cudaSuccess) return cuda_fail(c, e, "cudaMalloc touched list");
-        long long one = c->touched_count ? 1 : 0;
-        if ((e = grow(c->touched_count, one, 1)) != cudaSuccess) return cuda_fail(c, e, "cudaMalloc touched count");
         c->touched_cap = nb;
         c->grid_sparse_ok = false;
     }
@@ -423,11 +423,12 @@ int touched_buffers(tb_ctx* c, long long nb) {
 // caller's); the following steps of the same call zero only the node blocks
 // touched by this or the previous step, which are the only ones that can be
 // non-zero, so the grid matches the reference's dense fillzero!
-// (src/Core/zero.jl:100-106) at a fraction of the traffic. Nothing is cached
-// across calls: a later grid may reuse an earlier grid's address.
+// (src/Core/zero.jl:100-106) at a fraction of the traffic. The touched blocks
+// come from the scan of the step's binning (`touched`: it ran with touch_args).
+// Nothing is cached across calls: a later grid may reuse an earlier grid's address.
 template <int D, class T, int BW>
 cudaError_t p2g_with_zero(tb_ctx* c, const DMesh<D, T>& M, const PView<T>& P, const GView<T>& G,
-                          const Scalars<T>& S, const BinBuffers& B, const LaunchCfg& cfg) {
+                          const Scalars<T>& S, const BinBuffers& B, const LaunchCfg& cfg, bool touched) {
     if (G.bnum) {  // block-sparse grid: zero the stored nodes, scatter
         c->grid_sparse_ok = false;
         c->grid_zeroed = false;
@@ -438,20 +439,35 @@ cudaError_t p2g_with_zero(tb_ctx* c, const DMesh<D, T>& M, const PView<T>& P, co
     // after a grid half that zeroed its blocks once read, every P2G target is zero
     const bool zeroed = known && c->grid_zeroed;
     c->grid_zeroed = false;
-    std::swap(c->touched_cur, c->touched_prev);
-    cudaError_t e = cudaMemsetAsync(c->touched_cur, 0, size_t(M.nblocks), cfg.stream);
-    if (e == cudaSuccess && !known) e = cudaMemsetAsync(c->touched_prev, 0, size_t(M.nblocks), cfg.stream);
-    if (e == cudaSuccess) e = launch_mark_touched(D, M.nb, B, c->touched_cur, M.nblocks, cfg);
-    if (e == cudaSuccess)
-        e = launch_touched_list(c->touched_cur, c->touched_prev, M.nblocks, c->touched_list, c->touched_count, cfg);
-    if (e == cudaSuccess && !zeroed)
-        e = known ? launch_sparse_zero<D, T, BW>(M, G, c->touched_list, c->touched_count, cfg)
+    cudaError_t e = cudaSuccess;
+    if (!zeroed)
+        e = known ? launch_sparse_zero<D, T, BW>(M, G, c->touched_list, c->d_touched + c->touched_parity, cfg)
                   : launch_grid_zero<D, T>(M, G, cfg);
     if (e == cudaSuccess) e = launch_p2g<D, T, BW>(M, P, G, S, B, cfg);
     c->grid_key = G.m;
     c->grid_nblocks = M.nblocks;
-    c->grid_sparse_ok = (e == cudaSuccess);
+    c->grid_sparse_ok = (e == cudaSuccess) && touched;
     c->grid_dense_pending = !known;
+    return e;
+}
+
+// The touched-block pass of the next step's scan: the flags of the step before
+// become the previous ones, and the list length moves to the other counter (the
+// scan zeroes the one after it). `first`: no step of this call came before.
+cudaError_t touch_args(tb_ctx* c, const int* nb, long long nblocks, bool first, TouchArgs& t) {
+    cudaError_t e = cudaSuccess;
+    if (first) {
+        e = cudaMemsetAsync(c->touched_cur, 0, size_t(nblocks), c->stream);
+        if (e == cudaSuccess) e = cudaMemsetAsync(c->d_touched, 0, 2 * sizeof(int), c->stream);
+    }
+    std::swap(c->touched_cur, c->touched_prev);
+    c->touched_parity ^= 1;
+    t.cur = c->touched_cur;
+    t.prev = c->touched_prev;
+    t.list = c->touched_list;
+    t.count = c->d_touched + c->touched_parity;
+    t.next_count = c->d_touched + (c->touched_parity ^ 1);
+    t.nb = make_int3(nb[0], nb[1], nb[2]);
     return e;
 }
 
@@ -469,8 +485,8 @@ cudaError_t grid_update_sparse_or_dense(tb_ctx* c, const DMesh<D, T>& M, const G
     c->grid_dense_pending = false;
     c->grid_zeroed = false;
     if (known) {
-        const cudaError_t e = launch_sparse_grid_update<D, T, BW>(M, G, S, c->touched_cur, c->touched_list,
-                                                                  c->touched_count, cfg, zero_after);
+        const cudaError_t e = launch_sparse_grid_update<D, T, BW>(
+            M, G, S, c->touched_cur, c->touched_list, c->d_touched + c->touched_parity, cfg, zero_after);
         c->grid_zeroed = zero_after && e == cudaSuccess;
         return e;
     }
@@ -516,18 +532,26 @@ int run_step(tb_ctx* c, const tb_mesh* m, tb_particles* p, tb_partition* part, t
     SparseScratch SC{};
     if (G.bnum && do_bin && (rc = sparse_scratch(c, M.nblocks, SC)) != TB_OK) return rc;
     for (int s = 0; s < nsteps && e == cudaSuccess; ++s) {
+        const bool count_next = do_bin && do_g2p && s + 1 < nsteps;
+        // the touched node blocks matter to the steps after the first of a call
+        const bool touched = do_bin && do_p2g && nsteps > 1 && !G.bnum;
         if (do_bin) {
-            if (counted) e = launch_bin_rest(M.nblocks, P.n, B, cfg);
-            else e = x64 ? launch_bin<D, double>(M64, xs64, P.n, B, cfg) : launch_bin<D, T>(M, xs, P.n, B, cfg);
+            TouchArgs touch;
+            if (touched) e = touch_args(c, M.nb, M.nblocks, s == 0, touch);
+            if (e != cudaSuccess) break;
+            if (counted) e = launch_bin_rest(M.nblocks, P.n, B, cfg, touch, count_next);
+            else e = x64 ? launch_bin<D, double>(M64, xs64, P.n, B, cfg, touch, count_next)
+                         : launch_bin<D, T>(M, xs, P.n, B, cfg, touch, count_next);
             // a sparse grid follows the particles: update_sparsity! every step
             if (e == cudaSuccess && G.bnum)
                 e = launch_sparsity(D, M.nb, M.nblocks, B, SC, g->block_numbering, g->active_blocks, g->nactive, cfg);
         }
-        const bool count_next = do_bin && do_g2p && s + 1 < nsteps;
         counted = false;
         if (e == cudaSuccess && reorder) e = launch_reorder_score(RA, cfg);
         if (e == cudaSuccess && reorder) e = launch_reorder_apply(RA, fields.data(), int(fields.size()), cfg);
-        if (e == cudaSuccess && do_p2g) e = p2g_with_zero<D, T, BW>(c, M, P, G, S, B, cfg);
+        if (e == cudaSuccess && do_p2g && !do_bin)  // no binning zeroed it
+            e = cudaMemsetAsync(B.bnd_count, 0, sizeof(unsigned long long), cfg.stream);
+        if (e == cudaSuccess && do_p2g) e = p2g_with_zero<D, T, BW>(c, M, P, G, S, B, cfg, touched);
         if (e == cudaSuccess && do_grid)
             e = grid_update_sparse_or_dense<D, T, BW>(c, M, G, S, cfg, do_p2g && s + 1 < nsteps);
         if (e == cudaSuccess && do_g2p) {
@@ -941,7 +965,7 @@ int g2p2g_impl(tb_ctx* c, const tb_mesh* m, tb_particles* p, tb_partition* part,
     }
     c->grid_sparse_ok = false;  // dense zero and grid half, as the first step of a call
     if (e == cudaSuccess) e = launch_g2p<D, T, BW>(M, G, Pg, S, B, cfg, false);
-    if (e == cudaSuccess) e = p2g_with_zero<D, T, BW>(c, M, P, G, S, B, cfg);
+    if (e == cudaSuccess) e = p2g_with_zero<D, T, BW>(c, M, P, G, S, B, cfg, false);
     if (e == cudaSuccess) e = grid_update_sparse_or_dense<D, T, BW>(c, M, G, S, cfg);
     for (int d = 0; d < D && e == cudaSuccess; ++d) {
         void* dst = x64 ? static_cast<void*>(P.x64[d]) : static_cast<void*>(P.x[d]);
@@ -1331,13 +1355,15 @@ tb_ctx* tb_create(int32_t device, void* stream) {
         return nullptr;
     }
     cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, device);
-    if (cudaMalloc(&c->d_err, sizeof(int)) != cudaSuccess || cudaMalloc(&c->d_totals, 2 * sizeof(int)) != cudaSuccess ||
+    if (cudaMalloc(&c->d_err, sizeof(int)) != cudaSuccess || cudaMalloc(&c->d_totals, 32) != cudaSuccess ||
         cudaMallocHost(&c->h_totals, 2 * sizeof(int)) != cudaSuccess) {
         tb_destroy(c);
         return nullptr;
     }
     cudaMemset(c->d_err, 0, sizeof(int));
-    cudaMemset(c->d_totals, 0, 2 * sizeof(int));
+    cudaMemset(c->d_totals, 0, 32);
+    c->d_bnd = reinterpret_cast<unsigned long long*>(c->d_totals + 2);
+    c->d_touched = c->d_totals + 4;
     return c;
 }
 
@@ -1361,7 +1387,6 @@ void tb_destroy(tb_ctx* c) {
     cudaFree(c->touched_cur);
     cudaFree(c->touched_prev);
     cudaFree(c->touched_list);
-    cudaFree(c->touched_count);
     cudaFree(c->adj_grid);
     cudaFree(c->adj_coef);
     cudaFree(c->g2p2g_x);

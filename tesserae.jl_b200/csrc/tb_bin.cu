@@ -4,17 +4,16 @@
 // ascending, particle id ascending inside a block (cpu_block_strategy.jl:174-190).
 //
 //   count    one thread per particle: findblock, warp-aggregated count atomics
-//   scan     3 launches over packed (count | nonempty << 32) 64-bit sums: tile
-//            reduce, single-CTA spine, tile rescan writing offsets, cursors,
-//            the compacted block list and the totals [nactive, nassigned]
+//   scan     packed (count | nonempty << 32) 64-bit sums: offsets, cursors, the
+//            compacted block list and the totals [nactive, nassigned], and the
+//            node blocks the transfer touches; one launch up to 16 tiles of 1024
+//            blocks, a tile reduction before it above
 //   scatter  a warp takes 4 chunks of 32 ids and reserves one run per (chunk,
 //            distinct block) with a single atomic, writing the particles in lane order
 //   fixup    one warp per non-empty block: the block's segment is a set of runs,
-//            one per scatter warp (32 consecutive particle ids), each ascending;
-//            the runs are ranked by warp id and copied in order. Blocks of more
-//            than 64 runs are sorted by a second kernel (one CTA per block,
-//            bitonic in shared memory, or in a global scratch region for
-//            segments above 2048 runs).
+//            one per scatter chunk, each ascending; the runs are ranked by chunk id
+//            and copied in order; blocks of more than 128 runs by the CTA (bitonic
+//            in shared memory, or in a global scratch region above 2048 runs)
 // The result is deterministic regardless of atomic order.
 #include "tb_launch.cuh"
 
@@ -92,26 +91,32 @@ __global__ void __launch_bounds__(256) scan_reduce_kernel(const int* __restrict_
     if (threadIdx.x == 0) partials[blockIdx.x] = total;
 }
 
-// Exclusive scan of the tile partials in place (one CTA).
-__global__ void __launch_bounds__(256) scan_spine_kernel(unsigned long long* partials, int ntiles) {
+// Offsets, cursors, the compacted block list and the totals from the counts. A
+// CTA sums what lies before its own tile itself: the tile partials
+// (scan_reduce_kernel), or, with ONE, the counts (up to SCAN_ONE tiles a CTA reads
+// at most 60 counts per thread, which costs less than a second launch; a third
+// launch for the prefix of the partials was 2 us of every step).
+// With touch.cur it also marks the node blocks that this step's transfer reaches
+// (every block within one block per axis of one that holds particles) and lists
+// those marked now or in the previous transfer; the order of the list does not
+// matter. *touch.count must be zero; *touch.next_count is zeroed for the next
+// step, and *bnd_count for this one's P2G.
+template <bool ONE>
+__global__ void __launch_bounds__(256) scan_kernel(const int* __restrict__ counts, int nb,
+                                                   const unsigned long long* __restrict__ partials,
+                                                   int* __restrict__ offsets, int* __restrict__ cursors,
+                                                   int* __restrict__ blocklist, int* __restrict__ totals,
+                                                   unsigned long long* __restrict__ bnd_count, TouchArgs touch) {
     __shared__ unsigned long long wt[8];
-    unsigned long long carry = 0;
-    for (int c = 0; c < ntiles; c += 256) {
-        const int i = c + threadIdx.x;
-        unsigned long long v = i < ntiles ? partials[i] : 0ull;
-        unsigned long long total;
-        unsigned long long incl = block_incl_scan(v, wt, total);
-        if (i < ntiles) partials[i] = carry + incl - v;
-        carry += total;
+    const int tile0 = blockIdx.x * SCAN_TILE, base = tile0 + threadIdx.x * 4;
+    unsigned long long before = 0;
+    if constexpr (ONE) {
+        for (int b = threadIdx.x; b < tile0; b += 256) before += pack_count(counts[b]);
+    } else {
+        for (int t = threadIdx.x; t < int(blockIdx.x); t += 256) before += partials[t];
     }
-}
-
-__global__ void __launch_bounds__(256) scan_finalize_kernel(const int* __restrict__ counts, int nb,
-                                                            const unsigned long long* __restrict__ partials,
-                                                            int* __restrict__ offsets, int* __restrict__ cursors,
-                                                            int* __restrict__ blocklist, int* __restrict__ totals) {
-    __shared__ unsigned long long wt[8];
-    const int base = blockIdx.x * SCAN_TILE + threadIdx.x * 4;
+    unsigned long long prefix;
+    block_incl_scan(before, wt, prefix);
     int c[4];
     unsigned long long s = 0;
 #pragma unroll
@@ -121,7 +126,7 @@ __global__ void __launch_bounds__(256) scan_finalize_kernel(const int* __restric
     }
     unsigned long long total;
     unsigned long long incl = block_incl_scan(s, wt, total);
-    unsigned long long run = partials[blockIdx.x] + incl - s;  // exclusive prefix of this thread
+    unsigned long long run = prefix + incl - s;  // exclusive prefix of this thread
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         const int b = base + k;
@@ -137,6 +142,35 @@ __global__ void __launch_bounds__(256) scan_finalize_kernel(const int* __restric
                 totals[1] = int(run & 0xffffffffull);
             }
         }
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        if (bnd_count) *bnd_count = 0;
+        if (touch.next_count) *touch.next_count = 0;
+    }
+    if (!touch.cur) return;
+    const int lane = threadIdx.x & 31;
+#pragma unroll 1
+    for (int k = 0; k < 4; ++k) {
+        const int B = tile0 + k * 256 + threadIdx.x;  // neighbouring threads, neighbouring blocks
+        bool t = false;
+        if (B < nb) {
+            const int bx = B % touch.nb.x, by = (B / touch.nb.x) % touch.nb.y, bz = B / (touch.nb.x * touch.nb.y);
+            int any = 0;
+            for (int z = max(bz - 1, 0); z <= min(bz + 1, touch.nb.z - 1); ++z)
+                for (int y = max(by - 1, 0); y <= min(by + 1, touch.nb.y - 1); ++y) {
+                    const int* row = counts + touch.nb.x * (y + touch.nb.y * z);
+                    any |= row[bx];
+                    if (bx > 0) any |= row[bx - 1];
+                    if (bx + 1 < touch.nb.x) any |= row[bx + 1];
+                }
+            touch.cur[B] = any != 0;
+            t = any != 0 || touch.prev[B] != 0;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, t);
+        int at = 0;
+        if (lane == 0 && m) at = atomicAdd(touch.count, __popc(m));
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (t) touch.list[at + __popc(m & lanemask_lt())] = B;
     }
 }
 
@@ -204,269 +238,305 @@ __device__ __forceinline__ int fix_excl_scan(int v, int* wsum, int& total) {
     return wprefix + incl - v;
 }
 
-// Blocks of more than FIXW_RUNS runs, one CTA per block. Runs are found in
-// segment order, their keys (scatter warp id << 32 | run index) bitonic-sorted,
+// A block's segment of the scattered ids is a concatenation of runs, one per
+// scatter chunk (32 consecutive ids) that held particles of the block, each
+// ascending and contiguous, and no two runs of a segment share a chunk id.
+//
+// By a warp, up to FIXW_RUNS runs: the run heads are found with ballots, the runs
+// ranked by chunk id (every run against every run) and the segment copied
+// element-parallel, each element to its run's place.
+//
+// By the CTA, more runs: the keys (chunk id << 32 | run index) are bitonic-sorted,
 // the output start of each run is the prefix sum of the run lengths in sorted
-// order, and the segment is copied element-parallel (each element to its run's
-// place), all in shared memory when the padded key count fits; above that
-// (more than FIX_SMEM_KEYS runs) the keys are sorted in the block's own region
-// [2s, 2s + 2n) of the global scratch (next_pow2(k) <= 2n, segments disjoint)
-// and each thread copies whole runs.
-__global__ void __launch_bounds__(FIX_THREADS) bin_fixup_kernel(const int* __restrict__ totals,
-                                                                const int* __restrict__ blocklist,
-                                                                const int* __restrict__ offsets,
-                                                                const int* __restrict__ counts,
-                                                                const int* __restrict__ S, int* __restrict__ perm,
-                                                                unsigned long long* __restrict__ gscratch) {
-    __shared__ unsigned long long sbuf[FIX_SMEM_KEYS];
-    __shared__ int hpos[FIX_SMEM_KEYS + 1];  // run starts, segment order
-    __shared__ int hout[FIX_SMEM_KEYS];      // output start of each run, segment order
-    __shared__ int kcount;
-    __shared__ int wsum[FIX_THREADS / 32];
-    const int nactive = totals[0];
+// order, and the segment is copied element-parallel, all in shared memory when
+// the padded key count fits; above that (more than FIX_SMEM_KEYS runs) the keys
+// are sorted in the block's own region [2s, 2s + 2n) of the global scratch
+// (next_pow2(k) <= 2n, segments disjoint) and each thread copies whole runs.
+constexpr int FIXW_RUNS = 128;
+constexpr int FIXW_U = 8;  // chunks of 32 ids loaded together
+
+struct FixShared {
+    unsigned long long sbuf[FIX_SMEM_KEYS];
+    int hpos[FIX_SMEM_KEYS + 1];  // run starts, segment order
+    int hout[FIX_SMEM_KEYS];      // output start of each run, segment order
+    int kcount;
+    int wsum[FIX_THREADS / 32];
+    int over[FIX_THREADS / 32];  // this round's blocks with too many runs (-1: none)
+};
+
+// Segment S[s, s + n) to out, by the whole CTA.
+__device__ __forceinline__ void fixup_cta(FixShared& sm, const int* __restrict__ S, int s, int n,
+                                          int* __restrict__ perm, unsigned long long* __restrict__ gscratch) {
+    unsigned long long* sbuf = sm.sbuf;
+    int *hpos = sm.hpos, *hout = sm.hout, *wsum = sm.wsum;
+    int& kcount = sm.kcount;
     const int tid = threadIdx.x;
     auto is_head = [](const int* seg, int j, int v) { return j == 0 || (seg[j - 1] >> 5) != (v >> 5); };
-    for (int bi = blockIdx.x; bi < nactive; bi += gridDim.x) {
-        const int b = blocklist[bi] - 1;
-        const int s = offsets[b];
-        const int n = counts[b];
-        const int* seg = S + s;
-        int* out = perm + s;
-        // Run heads: the first element, and every element whose warp id differs
-        // from its predecessor's.
-        int myheads = 0;
-        for (int j = tid; j < n; j += FIX_THREADS) myheads += is_head(seg, j, seg[j]);
-        int k;
-        fix_excl_scan(myheads, wsum, k);
-        const int K = next_pow2(k);
-        if (K <= FIX_SMEM_KEYS) {
-            // 1. heads in segment order: positions and keys
-            int rbase = 0;
-            for (int j0 = 0; j0 < n; j0 += FIX_THREADS) {
-                const int j = j0 + tid;
-                const int v = j < n ? seg[j] : 0;
-                const int h = (j < n && is_head(seg, j, v)) ? 1 : 0;
-                int tot;
-                const int r = rbase + fix_excl_scan(h, wsum, tot);
-                if (h) {
-                    hpos[r] = j;
-                    sbuf[r] = ((unsigned long long)(unsigned)(v >> 5) << 32) | (unsigned)r;
-                }
-                rbase += tot;
+    const int* seg = S + s;
+    int* out = perm + s;
+    // Run heads: the first element, and every element whose warp id differs
+    // from its predecessor's.
+    int myheads = 0;
+    for (int j = tid; j < n; j += FIX_THREADS) myheads += is_head(seg, j, seg[j]);
+    int k;
+    fix_excl_scan(myheads, wsum, k);
+    const int K = next_pow2(k);
+    if (K <= FIX_SMEM_KEYS) {
+        // 1. heads in segment order: positions and keys
+        int rbase = 0;
+        for (int j0 = 0; j0 < n; j0 += FIX_THREADS) {
+            const int j = j0 + tid;
+            const int v = j < n ? seg[j] : 0;
+            const int h = (j < n && is_head(seg, j, v)) ? 1 : 0;
+            int tot;
+            const int r = rbase + fix_excl_scan(h, wsum, tot);
+            if (h) {
+                hpos[r] = j;
+                sbuf[r] = ((unsigned long long)(unsigned)(v >> 5) << 32) | (unsigned)r;
             }
-            if (tid == 0) hpos[k] = n;
-            for (int t = k + tid; t < K; t += FIX_THREADS) sbuf[t] = ~0ull;
-            __syncthreads();
-            // 2. bitonic sort of the K keys (ascending)
-            for (int size = 2; size <= K; size <<= 1) {
-                for (int stride = size >> 1; stride > 0; stride >>= 1) {
-                    for (int i = tid; i < (K >> 1); i += FIX_THREADS) {
-                        const int lo = (i / stride) * 2 * stride + (i % stride);
-                        const int hi = lo + stride;
-                        const bool asc = (lo & size) == 0;
-                        const unsigned long long a = sbuf[lo], c = sbuf[hi];
-                        if ((a > c) == asc) {
-                            sbuf[lo] = c;
-                            sbuf[hi] = a;
-                        }
-                    }
-                    __syncthreads();
-                }
-            }
-            // 3. output start of each run: lengths summed in sorted order
-            int obase = 0;
-            for (int i0 = 0; i0 < k; i0 += FIX_THREADS) {
-                const int i = i0 + tid;
-                int r = 0, len = 0;
-                if (i < k) {
-                    r = int(sbuf[i] & 0xffffffffull);
-                    len = hpos[r + 1] - hpos[r];
-                }
-                int tot;
-                const int st = obase + fix_excl_scan(len, wsum, tot);
-                if (i < k) hout[r] = st;
-                obase += tot;
-            }
-            __syncthreads();
-            // 4. element-parallel copy: an element's run is the number of heads at
-            //    or before it, minus one
-            rbase = 0;
-            for (int j0 = 0; j0 < n; j0 += FIX_THREADS) {
-                const int j = j0 + tid;
-                const int v = j < n ? seg[j] : 0;
-                const int h = (j < n && is_head(seg, j, v)) ? 1 : 0;
-                int tot;
-                const int r = rbase + fix_excl_scan(h, wsum, tot) + h - 1;
-                if (j < n) out[hout[r] + (j - hpos[r])] = v + 1;
-                rbase += tot;
-            }
-            __syncthreads();
-            continue;
+            rbase += tot;
         }
-        unsigned long long* buf = gscratch + 2ll * s;
-        if (tid == 0) kcount = 0;
+        if (tid == 0) hpos[k] = n;
+        for (int t = k + tid; t < K; t += FIX_THREADS) sbuf[t] = ~0ull;
         __syncthreads();
-        for (int j = tid; j < n; j += FIX_THREADS) {
-            const int v = seg[j];
-            if (is_head(seg, j, v)) {
-                const int idx = atomicAdd(&kcount, 1);
-                buf[idx] = ((unsigned long long)(unsigned)(v >> 5) << 32) | (unsigned)j;
-            }
-        }
-        __syncthreads();
-        for (int t = k + tid; t < K; t += FIX_THREADS) buf[t] = ~0ull;
-        __syncthreads();
-        // Bitonic sort of the K keys (ascending).
+        // 2. bitonic sort of the K keys (ascending)
         for (int size = 2; size <= K; size <<= 1) {
             for (int stride = size >> 1; stride > 0; stride >>= 1) {
                 for (int i = tid; i < (K >> 1); i += FIX_THREADS) {
                     const int lo = (i / stride) * 2 * stride + (i % stride);
                     const int hi = lo + stride;
                     const bool asc = (lo & size) == 0;
-                    const unsigned long long a = buf[lo], c = buf[hi];
+                    const unsigned long long a = sbuf[lo], c = sbuf[hi];
                     if ((a > c) == asc) {
-                        buf[lo] = c;
-                        buf[hi] = a;
+                        sbuf[lo] = c;
+                        sbuf[hi] = a;
                     }
                 }
                 __syncthreads();
             }
         }
-        // Copy the runs in sorted order; each run is at most 32 long.
-        int base = 0;
-        for (int c0 = 0; c0 < k; c0 += FIX_THREADS) {
-            const int r = c0 + tid;
-            int len = 0, j0 = 0;
-            if (r < k) {
-                const unsigned long long e = buf[r];
-                j0 = int(e & 0xffffffffull);
-                const int w = int(e >> 32);
-                len = 1;
-                while (j0 + len < n && (seg[j0 + len] >> 5) == w) ++len;
+        // 3. output start of each run: lengths summed in sorted order
+        int obase = 0;
+        for (int i0 = 0; i0 < k; i0 += FIX_THREADS) {
+            const int i = i0 + tid;
+            int r = 0, len = 0;
+            if (i < k) {
+                r = int(sbuf[i] & 0xffffffffull);
+                len = hpos[r + 1] - hpos[r];
             }
-            int total;
-            const int excl = base + fix_excl_scan(len, wsum, total);
-            for (int t = 0; t < len; ++t) out[excl + t] = seg[j0 + t] + 1;
-            base += total;
+            int tot;
+            const int st = obase + fix_excl_scan(len, wsum, tot);
+            if (i < k) hout[r] = st;
+            obase += tot;
+        }
+        __syncthreads();
+        // 4. element-parallel copy: an element's run is the number of heads at
+        //    or before it, minus one
+        rbase = 0;
+        for (int j0 = 0; j0 < n; j0 += FIX_THREADS) {
+            const int j = j0 + tid;
+            const int v = j < n ? seg[j] : 0;
+            const int h = (j < n && is_head(seg, j, v)) ? 1 : 0;
+            int tot;
+            const int r = rbase + fix_excl_scan(h, wsum, tot) + h - 1;
+            if (j < n) out[hout[r] + (j - hpos[r])] = v + 1;
+            rbase += tot;
+        }
+        __syncthreads();
+        return;
+    }
+    unsigned long long* buf = gscratch + 2ll * s;
+    if (tid == 0) kcount = 0;
+    __syncthreads();
+    for (int j = tid; j < n; j += FIX_THREADS) {
+        const int v = seg[j];
+        if (is_head(seg, j, v)) {
+            const int idx = atomicAdd(&kcount, 1);
+            buf[idx] = ((unsigned long long)(unsigned)(v >> 5) << 32) | (unsigned)j;
+        }
+    }
+    __syncthreads();
+    for (int t = k + tid; t < K; t += FIX_THREADS) buf[t] = ~0ull;
+    __syncthreads();
+    // Bitonic sort of the K keys (ascending).
+    for (int size = 2; size <= K; size <<= 1) {
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+            for (int i = tid; i < (K >> 1); i += FIX_THREADS) {
+                const int lo = (i / stride) * 2 * stride + (i % stride);
+                const int hi = lo + stride;
+                const bool asc = (lo & size) == 0;
+                const unsigned long long a = buf[lo], c = buf[hi];
+                if ((a > c) == asc) {
+                    buf[lo] = c;
+                    buf[hi] = a;
+                }
+            }
+            __syncthreads();
+        }
+    }
+    // Copy the runs in sorted order; each run is at most 32 long.
+    int base = 0;
+    for (int c0 = 0; c0 < k; c0 += FIX_THREADS) {
+        const int r = c0 + tid;
+        int len = 0, j0 = 0;
+        if (r < k) {
+            const unsigned long long e = buf[r];
+            j0 = int(e & 0xffffffffull);
+            const int w = int(e >> 32);
+            len = 1;
+            while (j0 + len < n && (seg[j0 + len] >> 5) == w) ++len;
+        }
+        int total;
+        const int excl = base + fix_excl_scan(len, wsum, total);
+        for (int t = 0; t < len; ++t) out[excl + t] = seg[j0 + t] + 1;
+        base += total;
+    }
+    __syncthreads();
+}
+
+// Segment S[s, s + n) to out, by one warp with its own shared arrays; false (and
+// nothing written) if it has more than FIXW_RUNS runs.
+__device__ __forceinline__ bool fixup_warp(int* hpos, int* hkey, int* hout, const int* __restrict__ seg, int n,
+                                           int* __restrict__ out) {
+    const int lane = threadIdx.x & 31;
+    const unsigned full = 0xffffffffu, below = (1u << lane) - 1u;
+    // A run is at most 32 long, so a longer segment has too many runs: hand it
+    // over without walking it, and stop walking at the first run past the limit.
+    if (n > FIXW_RUNS * 32) return false;
+    int nruns = 0;
+    // The segment is read FIXW_U chunks of 32 at a time, all loads of a batch
+    // issued before any is used; the predecessor of a chunk's first element
+    // is lane 31 of the chunk before.
+    int last = -1;
+    for (int J0 = 0; J0 < n && nruns <= FIXW_RUNS; J0 += 32 * FIXW_U) {
+        int vv[FIXW_U];
+#pragma unroll
+        for (int u = 0; u < FIXW_U; ++u) {
+            const int j = J0 + 32 * u + lane;
+            vv[u] = j < n ? seg[j] : 0;
+        }
+#pragma unroll
+        for (int u = 0; u < FIXW_U; ++u) {
+            const int j0 = J0 + 32 * u;
+            if (j0 >= n) break;
+            const int j = j0 + lane, v = vv[u];
+            int prev = __shfl_up_sync(full, v, 1);
+            if (lane == 0) prev = last;
+            last = __shfl_sync(full, v, 31);
+            const bool head = j < n && (j == 0 || (prev >> 5) != (v >> 5));
+            const unsigned hm = __ballot_sync(full, head);
+            const int idx = nruns + __popc(hm & below);
+            if (head && idx < FIXW_RUNS) {
+                hpos[idx] = j;
+                hkey[idx] = v >> 5;
+            }
+            nruns += __popc(hm);
+        }
+    }
+    if (nruns > FIXW_RUNS) return false;
+    if (lane == 0) hpos[nruns] = n;
+    __syncwarp();
+    // output start of each run: total length of the runs with a smaller chunk id
+    for (int r = lane; r < nruns; r += 32) {
+        const int key = hkey[r];
+        int start = 0, at = hpos[0];
+        for (int q = 0; q < nruns; ++q) {
+            const int next = hpos[q + 1];
+            if (hkey[q] < key) start += next - at;
+            at = next;
+        }
+        hout[r] = start;
+    }
+    __syncwarp();
+    // copy element-parallel: the run of element j is the number of heads at
+    // or before j, minus one
+    int rbase = 0;
+    last = -1;
+    for (int J0 = 0; J0 < n; J0 += 32 * FIXW_U) {
+        int vv[FIXW_U];
+#pragma unroll
+        for (int u = 0; u < FIXW_U; ++u) {
+            const int j = J0 + 32 * u + lane;
+            vv[u] = j < n ? seg[j] : 0;
+        }
+#pragma unroll
+        for (int u = 0; u < FIXW_U; ++u) {
+            const int j0 = J0 + 32 * u;
+            if (j0 >= n) break;
+            const int j = j0 + lane, v = vv[u];
+            int prev = __shfl_up_sync(full, v, 1);
+            if (lane == 0) prev = last;
+            last = __shfl_sync(full, v, 31);
+            const bool head = j < n && (j == 0 || (prev >> 5) != (v >> 5));
+            const unsigned hm = __ballot_sync(full, head);
+            const int r = rbase + __popc(hm & (below | (1u << lane))) - 1;
+            if (j < n) out[hout[r] + (j - hpos[r])] = v + 1;
+            rbase += __popc(hm);
+        }
+    }
+    __syncwarp();
+    return true;
+}
+
+// A CTA takes 8 blocks of the list at a time, one per warp, and then together
+// those that a warp could not do; one block at a time in crowded scenes (1024
+// particles or more per block on average, whose blocks mostly have too many runs),
+// fewer than 8 where there are too few blocks to give every CTA 8 (a 74 k particle
+// sphere of 27 per cell, most blocks over the limit: 0.31 ms per two steps at one
+// block per CTA, 0.40 at eight).
+// One launch: as two (warps, then the blocks they listed) the second cost 2 us of
+// every step. With `zero`, the counts of all blocks are zeroed (the next step's
+// G2P counts into them).
+__global__ void __launch_bounds__(FIX_THREADS) bin_fixup_kernel(const int* __restrict__ totals,
+                                                                const int* __restrict__ blocklist,
+                                                                const int* __restrict__ offsets,
+                                                                const int* __restrict__ S, int* __restrict__ perm,
+                                                                unsigned long long* __restrict__ gscratch,
+                                                                int* __restrict__ zero, int nb) {
+    constexpr int NWARP = FIX_THREADS / 32;
+    __shared__ FixShared sm;
+    __shared__ int whpos[NWARP][FIXW_RUNS + 1], whkey[NWARP][FIXW_RUNS], whout[NWARP][FIXW_RUNS];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int nactive = totals[0];
+    const int take = (nactive > 0 && totals[1] / nactive >= 1024)
+                         ? 1
+                         : min(NWARP, (nactive + int(gridDim.x) - 1) / int(gridDim.x));
+    for (int b0 = blockIdx.x * take; b0 < nactive; b0 += gridDim.x * take) {
+        int over = -1;
+        if (w < take && b0 + w < nactive) {
+            const int b = blocklist[b0 + w] - 1, s = offsets[b];
+            if (!fixup_warp(whpos[w], whkey[w], whout[w], S + s, offsets[b + 1] - s, perm + s)) over = b;
+        }
+        if (lane == 0) sm.over[w] = over;
+        __syncthreads();
+        for (int q = 0; q < take; ++q) {
+            const int b = sm.over[q];  // uniform over the CTA
+            if (b >= 0) fixup_cta(sm, S, offsets[b], offsets[b + 1] - offsets[b], perm, gscratch);
         }
         __syncthreads();
     }
-}
-
-// One warp per non-empty block: the block's segment of the scattered ids is a
-// concatenation of runs, one per scatter warp that held particles of the block,
-// each ascending and contiguous, and no two runs of a segment share a warp id.
-// The warp finds the run heads with ballots, ranks the runs by warp id (every
-// run against every run, at most FIXW_RUNS of them) and copies the segment
-// element-parallel, each element to its run's place. A block with more runs is appended to an
-// overflow list that bin_fixup_kernel then sorts.
-constexpr int FIXW_RUNS = 64;
-constexpr int FIXW_U = 8;  // chunks of 32 ids loaded together
-constexpr int FIXW_THREADS = 256;
-
-__global__ void __launch_bounds__(FIXW_THREADS) bin_fixup_warp_kernel(const int* __restrict__ totals,
-                                                                      const int* __restrict__ blocklist,
-                                                                      const int* __restrict__ offsets,
-                                                                      const int* __restrict__ counts,
-                                                                      const int* __restrict__ S,
-                                                                      int* __restrict__ perm,
-                                                                      int* __restrict__ overflow,
-                                                                      unsigned long long* __restrict__ noverflow) {
-    constexpr int NWARP = FIXW_THREADS / 32;
-    __shared__ int hpos[NWARP][FIXW_RUNS + 1];
-    __shared__ int hkey[NWARP][FIXW_RUNS];
-    __shared__ int hout[NWARP][FIXW_RUNS];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int nactive = totals[0];
-    const unsigned full = 0xffffffffu;
-    const unsigned below = (1u << lane) - 1u;
-    for (int bi = blockIdx.x * NWARP + w; bi < nactive; bi += gridDim.x * NWARP) {
-        const int b = blocklist[bi] - 1;
-        const int s = offsets[b], n = counts[b];
-        const int* seg = S + s;
-        int* out = perm + s;
-        int nruns = 0;
-        // A run is at most 32 long, so a longer segment has too many runs: hand it
-        // over without walking it (one warp reading thousands of ids serially was
-        // most of the fix-up time of crowded scenes), and stop walking at the
-        // first run past the limit.
-        if (n > FIXW_RUNS * 32) nruns = FIXW_RUNS + 1;
-        // The segment is read FIXW_U chunks of 32 at a time, all loads of a batch
-        // issued before any is used; the predecessor of a chunk's first element
-        // is lane 31 of the chunk before.
-        int last = -1;
-        for (int J0 = 0; J0 < n && nruns <= FIXW_RUNS; J0 += 32 * FIXW_U) {
-            int vv[FIXW_U];
-#pragma unroll
-            for (int u = 0; u < FIXW_U; ++u) {
-                const int j = J0 + 32 * u + lane;
-                vv[u] = j < n ? seg[j] : 0;
-            }
-#pragma unroll
-            for (int u = 0; u < FIXW_U; ++u) {
-                const int j0 = J0 + 32 * u;
-                if (j0 >= n) break;
-                const int j = j0 + lane, v = vv[u];
-                int prev = __shfl_up_sync(full, v, 1);
-                if (lane == 0) prev = last;
-                last = __shfl_sync(full, v, 31);
-                const bool head = j < n && (j == 0 || (prev >> 5) != (v >> 5));
-                const unsigned hm = __ballot_sync(full, head);
-                const int idx = nruns + __popc(hm & below);
-                if (head && idx < FIXW_RUNS) {
-                    hpos[w][idx] = j;
-                    hkey[w][idx] = v >> 5;
-                }
-                nruns += __popc(hm);
-            }
-        }
-        if (nruns > FIXW_RUNS) {
-            if (lane == 0) overflow[atomicAdd(noverflow, 1ull)] = b + 1;
-            __syncwarp();
-            continue;
-        }
-        if (lane == 0) hpos[w][nruns] = n;
-        __syncwarp();
-        // output start of each run: total length of the runs with a smaller warp id
-        for (int r = lane; r < nruns; r += 32) {
-            const int key = hkey[w][r];
-            int start = 0;
-            for (int q = 0; q < nruns; ++q)
-                if (hkey[w][q] < key) start += hpos[w][q + 1] - hpos[w][q];
-            hout[w][r] = start;
-        }
-        __syncwarp();
-        // copy element-parallel: the run of element j is the number of heads at
-        // or before j, minus one
-        int rbase = 0;
-        last = -1;
-        for (int J0 = 0; J0 < n; J0 += 32 * FIXW_U) {
-            int vv[FIXW_U];
-#pragma unroll
-            for (int u = 0; u < FIXW_U; ++u) {
-                const int j = J0 + 32 * u + lane;
-                vv[u] = j < n ? seg[j] : 0;
-            }
-#pragma unroll
-            for (int u = 0; u < FIXW_U; ++u) {
-                const int j0 = J0 + 32 * u;
-                if (j0 >= n) break;
-                const int j = j0 + lane, v = vv[u];
-                int prev = __shfl_up_sync(full, v, 1);
-                if (lane == 0) prev = last;
-                last = __shfl_sync(full, v, 31);
-                const bool head = j < n && (j == 0 || (prev >> 5) != (v >> 5));
-                const unsigned hm = __ballot_sync(full, head);
-                const int r = rbase + __popc(hm & (below | (1u << lane))) - 1;
-                if (j < n) out[hout[w][r] + (j - hpos[w][r])] = v + 1;
-                rbase += __popc(hm);
-            }
-        }
-        __syncwarp();
-    }
+    if (zero)
+        for (int b = blockIdx.x * FIX_THREADS + threadIdx.x; b < nb; b += gridDim.x * FIX_THREADS) zero[b] = 0;
 }
 
 inline unsigned grid_for(long long n, int threads) { return unsigned((n + threads - 1) / threads); }
+
+constexpr int SCAN_ONE = 16;  // tiles up to which the scan is one launch
+
+void launch_scan(const int* counts, int nb, unsigned long long* partials, int* offsets, int* cursors, int* blocklist,
+                 int* totals, unsigned long long* bnd_count, const TouchArgs& touch, const LaunchCfg& cfg) {
+    const int nt = scan_tiles(nb);
+    if (nt <= SCAN_ONE) {
+        scan_kernel<true><<<nt, 256, 0, cfg.stream>>>(counts, nb, partials, offsets, cursors, blocklist, totals,
+                                                      bnd_count, touch);
+        ++*cfg.launches;
+        return;
+    }
+    scan_reduce_kernel<<<nt, 256, 0, cfg.stream>>>(counts, nb, partials);
+    scan_kernel<false><<<nt, 256, 0, cfg.stream>>>(counts, nb, partials, offsets, cursors, blocklist, totals, bnd_count,
+                                                   touch);
+    *cfg.launches += 2;
+}
 
 // ---- sparse grid numbering ----------------------------------------------
 // act[B] = 1 for every node block B within one block per axis of a block that
@@ -512,14 +582,10 @@ cudaError_t launch_sparsity(int dim, const int* nbv, int nblocks, const BinBuffe
     if (dim == 3) sparse_mark_kernel<3><<<mgrid, 128, 0, cfg.stream>>>(b.totals, b.blocklist, nb, sc.act);
     else sparse_mark_kernel<2><<<mgrid, 128, 0, cfg.stream>>>(b.totals, b.blocklist, nb, sc.act);
     // the binning's scan over the activity: offsets = ranks, blocklist = the active list
-    const int nt = scan_tiles(nblocks);
-    scan_reduce_kernel<<<nt, 256, 0, cfg.stream>>>(sc.act, nblocks, sc.partials);
-    scan_spine_kernel<<<1, 256, 0, cfg.stream>>>(sc.partials, nt);
-    scan_finalize_kernel<<<nt, 256, 0, cfg.stream>>>(sc.act, nblocks, sc.partials, sc.offsets, sc.cursors, blist,
-                                                     sc.totals);
+    launch_scan(sc.act, nblocks, sc.partials, sc.offsets, sc.cursors, blist, sc.totals, nullptr, TouchArgs{}, cfg);
     sparse_number_kernel<<<std::max(1, std::min((nblocks + 255) / 256, cfg.num_sms * 8)), 256, 0, cfg.stream>>>(
         sc.act, sc.offsets, nblocks, sc.totals, bnum, nact);
-    *cfg.launches += 5;
+    *cfg.launches += 2;
     return cudaGetLastError();
 }
 
@@ -537,50 +603,38 @@ cudaError_t launch_bin_count(const DMesh<D, T>& M, const T* const* x, long long 
     return cudaGetLastError();
 }
 
-cudaError_t launch_bin_rest(int nb, long long n, const BinBuffers& b, const LaunchCfg& cfg) {
-    const int nt = scan_tiles(nb);
+cudaError_t launch_bin_rest(int nb, long long n, const BinBuffers& b, const LaunchCfg& cfg, const TouchArgs& touch,
+                            bool zero_counts) {
     {
         KernelScope ks(cfg, "bin_scan");
-        scan_reduce_kernel<<<nt, 256, 0, cfg.stream>>>(b.counts, nb, b.partials);
-        scan_spine_kernel<<<1, 256, 0, cfg.stream>>>(b.partials, nt);
-        scan_finalize_kernel<<<nt, 256, 0, cfg.stream>>>(b.counts, nb, b.partials, b.offsets, b.cursors, b.blocklist,
-                                                         b.totals);
+        launch_scan(b.counts, nb, b.partials, b.offsets, b.cursors, b.blocklist, b.totals, b.bnd_count, touch, cfg);
     }
-    *cfg.launches += 3;
     if (n > 0) {
         {
             KernelScope ks(cfg, "bin_scatter");
             bin_scatter_kernel<<<grid_for(n, 256 * SCAT_IT), 256, 0, cfg.stream>>>(b.blockids, n, b.cursors,
                                                                                   b.perm_tmp);
         }
-        // Blocks of more than FIXW_RUNS runs go to an overflow list kept in the
-        // cursor array (free once the scatter is done), its length in partials[0].
-        cudaError_t e = cudaMemsetAsync(b.partials, 0, sizeof(unsigned long long), cfg.stream);
-        if (e != cudaSuccess) return e;
         KernelScope ks(cfg, "bin_fixup");
-        const int wgrid = std::max(1, std::min((nb + FIXW_THREADS / 32 - 1) / (FIXW_THREADS / 32), cfg.num_sms * 8));
-        bin_fixup_warp_kernel<<<wgrid, FIXW_THREADS, 0, cfg.stream>>>(b.totals, b.blocklist, b.offsets, b.counts,
-                                                                      b.perm_tmp, b.perm, b.cursors, b.partials);
-        const int grid = std::min(nb, cfg.num_sms * 16);
-        bin_fixup_kernel<<<grid, FIX_THREADS, 0, cfg.stream>>>(reinterpret_cast<const int*>(b.partials), b.cursors,
-                                                               b.offsets, b.counts, b.perm_tmp, b.perm,
-                                                               b.sort_scratch);
-        *cfg.launches += 3;
+        const int grid = std::max(1, std::min(nb, cfg.num_sms * 5));
+        bin_fixup_kernel<<<grid, FIX_THREADS, 0, cfg.stream>>>(b.totals, b.blocklist, b.offsets, b.perm_tmp, b.perm,
+                                                               b.sort_scratch, zero_counts ? b.counts : nullptr, nb);
+        *cfg.launches += 2;
     }
     return cudaGetLastError();
 }
 
 template <int D, class T>
 cudaError_t launch_bin(const DMesh<D, T>& M, const T* const* x, long long n, const BinBuffers& b,
-                       const LaunchCfg& cfg, bool) {
+                       const LaunchCfg& cfg, const TouchArgs& touch, bool zero_counts) {
     cudaError_t e = launch_bin_count<D, T>(M, x, n, b, cfg);
     if (e != cudaSuccess) return e;
-    return launch_bin_rest(M.nblocks, n, b, cfg);
+    return launch_bin_rest(M.nblocks, n, b, cfg, touch, zero_counts);
 }
 
 #define TB_INST_BIN(D, T)                                                                                     \
     template cudaError_t launch_bin<D, T>(const DMesh<D, T>&, const T* const*, long long, const BinBuffers&, \
-                                          const LaunchCfg&, bool);                                            \
+                                          const LaunchCfg&, const TouchArgs&, bool);                          \
     template cudaError_t launch_bin_count<D, T>(const DMesh<D, T>&, const T* const*, long long,              \
                                                 const BinBuffers&, const LaunchCfg&);
 TB_INST_BIN(3, double)

@@ -18,6 +18,18 @@ struct BinBuffers {
     unsigned long long* partials;  // [ntiles] scratch
     unsigned long long* sort_scratch;  // [2n] scratch for large blocks
     int* totals;          // [2] device: nactive, nassigned
+    unsigned long long* bnd_count;  // [1] blocks P2G leaves to its second launch; zeroed by every binning
+};
+
+// Node blocks that a step's transfer touches, found by the scan of its binning:
+// flags of this and the previous transfer, the list of blocks with either set.
+struct TouchArgs {
+    unsigned char* cur = nullptr;         // [nb]; null: not wanted
+    const unsigned char* prev = nullptr;  // [nb]
+    int* list = nullptr;                  // [nb]
+    int* count = nullptr;                 // [1] zero on entry
+    int* next_count = nullptr;            // [1] zeroed (the next step's count)
+    int3 nb = {1, 1, 1};                  // blocks per axis
 };
 
 // Scratch of a sparse grid's numbering pass (one int per block each, the scan
@@ -63,14 +75,16 @@ struct KernelScope {
 
 template <int D, class T>
 cudaError_t launch_bin(const DMesh<D, T>& M, const T* const* x, long long n, const BinBuffers& b,
-                       const LaunchCfg& cfg, bool count_only_done = false);
+                       const LaunchCfg& cfg, const TouchArgs& touch = TouchArgs{}, bool zero_counts = false);
 
 // Count kernel alone (positions -> blockids, counts); the rest of the pass in
 // launch_bin_rest. Split so a fused step can count inside G2P.
 template <int D, class T>
 cudaError_t launch_bin_count(const DMesh<D, T>& M, const T* const* x, long long n, const BinBuffers& b,
                              const LaunchCfg& cfg);
-cudaError_t launch_bin_rest(int nblocks, long long n, const BinBuffers& b, const LaunchCfg& cfg);
+// `zero_counts`: b.counts are zero again afterwards (for a G2P that counts ahead).
+cudaError_t launch_bin_rest(int nblocks, long long n, const BinBuffers& b, const LaunchCfg& cfg,
+                            const TouchArgs& touch = TouchArgs{}, bool zero_counts = false);
 
 // update_sparsity! from a binning pass: the node blocks within one block of a
 // block that holds particles (b.blocklist / b.totals), numbered in ascending
@@ -91,20 +105,14 @@ template <int D, class T>
 cudaError_t launch_grid_zero(const DMesh<D, T>& M, const GView<T>& G, const LaunchCfg& cfg);
 
 // With `count_next`, G2P also writes every moved particle's block id for the
-// next step into b.blockids and adds it to b.counts (which the caller zeroes
-// first): the count pass of the next step's binning, so that step runs
+// next step into b.blockids and adds it to b.counts (zeroed by this step's
+// binning): the count pass of the next step's binning, so that step runs
 // launch_bin_rest only.
 template <int D, class T, int BW>
 cudaError_t launch_g2p(const DMesh<D, T>& M, const GView<T>& G, const PView<T>& P, const Scalars<T>& s,
                        const BinBuffers& b, const LaunchCfg& cfg, bool count_next = false);
 
-// Sparse grid maintenance over node blocks touched now (cur) or in the previous
-// transfer (prev): see tb_transfer.cu.
-cudaError_t launch_mark_touched(int dim, const int* nbv, const BinBuffers& b, unsigned char* cur, int nblocks,
-                                const LaunchCfg& cfg);
-// The node blocks with cur or prev set, compacted into list[0 .. *count).
-cudaError_t launch_touched_list(const unsigned char* cur, const unsigned char* prev, int nblocks, int* list,
-                                int* count, const LaunchCfg& cfg);
+// Grid maintenance over the listed node blocks (TouchArgs): see tb_transfer.cu.
 template <int D, class T, int BW>
 cudaError_t launch_sparse_zero(const DMesh<D, T>& M, const GView<T>& G, const int* list, const int* count,
                                const LaunchCfg& cfg);
@@ -177,7 +185,6 @@ struct ReorderArgs {
     int nblocks;
     int* blockids;         // [n] permuted with the particles
     int* perm;             // [n] 1-based block-sorted permutation; identity after a reorder
-    const int* counts;     // [nblocks]
     const int* offsets;    // [nblocks + 1]
     double threshold;      // reorder when the score is below it (always at >= 1, never at <= 0)
     unsigned long long* acc;  // [2] scratch: same-block neighbours, non-empty blocks

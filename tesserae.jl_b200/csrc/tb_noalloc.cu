@@ -79,6 +79,7 @@ int run(const tb_mesh* m, const tb_particles* p, tb_partition* part, cudaStream_
     B.partials = reinterpret_cast<unsigned long long*>(scratch + kOffPartials);
     B.sort_scratch = reinterpret_cast<unsigned long long*>(scratch + kOffSort);
     B.totals = reinterpret_cast<int*>(scratch + kOffTotals);
+    B.bnd_count = reinterpret_cast<unsigned long long*>(scratch + kOffTotals + 16);
     int device = 0;
     cudaGetDevice(&device);
     int sms = 148;

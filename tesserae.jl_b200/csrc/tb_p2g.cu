@@ -637,10 +637,12 @@ struct PairAcc {
 // accumulators) in registers. Per record a lane loads the record once and
 // evaluates the x and y jets once for 9 nodes instead of 3, so the per-record
 // overhead (loads, jets, row factors) is paid 3 times per particle instead of
-// 9; the 25 pencils x 3 z-slots are 75 lanes of the 128-thread CTA. Blocks at the
-// mesh boundary run the same way (bspline_start), their partials summed in FP64.
-// With `bnd` given (KernelCorrection) every block whose halo tile leaves the mesh
-// is appended there instead, for a launch with full records.
+// 9; the 25 pencils x 3 z-slots are 75 lanes of the 128-thread CTA.
+// FULL: blocks at the mesh boundary run the same way (bspline_start), their
+// partials summed in FP64. Otherwise every block whose halo tile leaves the mesh is
+// appended to `bnd` for a launch with full records: the second gather costs the
+// interior blocks 2.6% (cube3d, 16.8 M particles: 1.047 against 1.020 ms), a second
+// launch 2 us.
 constexpr int PLANE_THREADS = 128;
 constexpr int PLANE_NR = 512;
 constexpr int CRS = 14;  // words of a PairRec record
@@ -686,7 +688,7 @@ __device__ __forceinline__ void accumulate_plane(const PairRec& o, const SlotPol
     }
 }
 
-template <bool X64>
+template <bool X64, bool FULL>
 __global__ void __launch_bounds__(PLANE_THREADS, 3)
     p2g_plane_kernel(DMesh<3, float> M, PView<float> P, GView<float> G, Scalars<float> s,
                      const int* __restrict__ totals, const int* __restrict__ blocklist,
@@ -736,9 +738,11 @@ __global__ void __launch_bounds__(PLANE_THREADS, 3)
                 interior = interior && org[d] >= 0 && org[d] + TS - 1 <= M.n[d] - 1;
             }
         }
-        if (bnd && !interior) {  // the full-record launch's block (uniform over the CTA)
-            if (tid == 0 && piece == 0) bnd[atomicAdd(bnd_count, 1ull)] = b;
-            continue;
+        if constexpr (!FULL) {
+            if (!interior) {  // the full-record launch's block (uniform over the CTA)
+                if (tid == 0 && piece == 0) bnd[atomicAdd(bnd_count, 1ull)] = b;
+                continue;
+            }
         }
         const int s0 = offsets[b], s1 = offsets[b + 1];
         const BlockPasses bp(s0, s1, per);
@@ -919,8 +923,12 @@ __global__ void __launch_bounds__(PLANE_THREADS, 3)
                     grid_add<3>(G, M, err, nx, ny, nz, val);
                 }
             };
-            if (interior) gather(0.0f, std::false_type{});
-            else gather(0.0, std::true_type{});
+            if constexpr (FULL) {
+                if (interior) gather(0.0f, std::false_type{});
+                else gather(0.0, std::true_type{});
+            } else {
+                gather(0.0f, std::false_type{});
+            }
         }
     }
 }
@@ -931,11 +939,11 @@ size_t plane_smem_bytes() {
            sizeof(int) * size_t(SH::NG + SH::NG + 1 + 32);
 }
 
-template <bool X64>
+template <bool X64, bool FULL>
 cudaError_t launch_plane(const DMesh<3, float>& M, const PView<float>& P, const GView<float>& G,
                          const Scalars<float>& s, const BinBuffers& b, const LaunchCfg& cfg, int* bnd,
                          unsigned long long* bnd_count) {
-    auto kern = p2g_plane_kernel<X64>;
+    auto kern = p2g_plane_kernel<X64, FULL>;
     const size_t smem = plane_smem_bytes();
     int grid = 0;
     cudaError_t e = prepare_launch(kern, PLANE_THREADS, smem, cfg, M.nblocks, grid);
@@ -1288,11 +1296,13 @@ cudaError_t launch_p2g_2d(const DMesh<2, T>& M, const PView<T>& P, const GView<T
 }
 
 
+constexpr int PLANE_ONE_BLOCKS = 16384;  // a 100^3-cell mesh
+
 // 3D. The quadratic B-spline in the FP32 forms takes the plane kernel (short
 // records, 9 nodes per lane). KernelCorrection changes the weights of cut windows
 // only: its interior blocks are plain B-spline, the others (their list in binning
-// scratch that is free until the next binning: one int per block in the cursors,
-// the count in the first scan partial) take full records.
+// scratch that is free until the next binning: one int per block in the cursors)
+// take full records.
 template <class T, bool X64>
 cudaError_t launch_p2g_3d(const DMesh<3, T>& M, const PView<T>& P, const GView<T>& G, const Scalars<T>& s,
                           const BinBuffers& b, const LaunchCfg& cfg) {
@@ -1303,12 +1313,15 @@ cudaError_t launch_p2g_3d(const DMesh<3, T>& M, const PView<T>& P, const GView<T
                    : launch_pencil<T, X64, P_APIC>(M, P, G, s, b, cfg);
     if (wls) return launch_pencil<T, X64, P_WLS>(M, P, G, s, b, cfg);
     if constexpr (sizeof(T) == 4) {
-        if (s.basis == TB_BSPLINE_QUADRATIC) return launch_plane<X64>(M, P, G, s, b, cfg, nullptr, nullptr);
-        if (s.basis == TB_KC_BSPLINE_QUADRATIC) {
-            cudaError_t e = cudaMemsetAsync(b.partials, 0, sizeof(unsigned long long), cfg.stream);
-            if (e == cudaSuccess) e = launch_plane<X64>(M, P, G, s, b, cfg, b.cursors, b.partials);
+        // one launch where it is worth its 2 us: P2G takes 2.6% less with two, which
+        // is 2 us from about 1 M particles on; up to PLANE_ONE_BLOCKS mesh blocks a
+        // B-spline takes one
+        if (s.basis == TB_BSPLINE_QUADRATIC && M.nblocks <= PLANE_ONE_BLOCKS)
+            return launch_plane<X64, true>(M, P, G, s, b, cfg, nullptr, nullptr);
+        if (s.basis == TB_BSPLINE_QUADRATIC || s.basis == TB_KC_BSPLINE_QUADRATIC) {
+            const cudaError_t e = launch_plane<X64, false>(M, P, G, s, b, cfg, b.cursors, b.bnd_count);
             if (e != cudaSuccess) return e;
-            return launch_pencil<T, X64, P_JET>(M, P, G, s, b, cfg, b.cursors, b.partials);
+            return launch_pencil<T, X64, P_JET>(M, P, G, s, b, cfg, b.cursors, b.bnd_count);
         }
     } else if (s.basis == TB_BSPLINE_QUADRATIC) {
         return launch_pencil<T, X64, P_BSP>(M, P, G, s, b, cfg);

@@ -24,7 +24,7 @@ constexpr int RO_THREADS = 256;
 // nassigned = offsets[nb]; nactive = number of non-empty blocks. Both come from
 // the partition arrays themselves, so the partition may come from any binning.
 __global__ void __launch_bounds__(RO_THREADS) reorder_score_kernel(const int* __restrict__ blockids, long long n,
-                                                                   const int* __restrict__ counts, int nb,
+                                                                   const int* __restrict__ offsets, int nb,
                                                                    unsigned long long* __restrict__ acc) {
     unsigned long long same = 0, active = 0;
     const long long stride = (long long)gridDim.x * blockDim.x;
@@ -32,7 +32,7 @@ __global__ void __launch_bounds__(RO_THREADS) reorder_score_kernel(const int* __
         const int a = blockids[p];
         same += (a != 0 && a == blockids[p + 1]);
     }
-    for (long long b = (long long)blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += stride) active += counts[b] > 0;
+    for (long long b = (long long)blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += stride) active += offsets[b + 1] > offsets[b];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         same += __shfl_down_sync(0xffffffffu, same, o);
@@ -93,7 +93,7 @@ cudaError_t launch_reorder_score(const ReorderArgs& a, const LaunchCfg& cfg) {
     const int grid = int(std::max<long long>(1, std::min<long long>((work + RO_THREADS - 1) / RO_THREADS,
                                                                     (long long)cfg.num_sms * 8)));
     KernelScope ks(cfg, "reorder_score");
-    reorder_score_kernel<<<grid, RO_THREADS, 0, cfg.stream>>>(a.blockids, a.n, a.counts, a.nblocks, a.acc);
+    reorder_score_kernel<<<grid, RO_THREADS, 0, cfg.stream>>>(a.blockids, a.n, a.offsets, a.nblocks, a.acc);
     reorder_decide_kernel<<<1, 1, 0, cfg.stream>>>(a.acc, a.offsets, a.nblocks, a.n, a.threshold, a.decision,
                                                    a.score, a.report_outside ? cfg.err : nullptr);
     *cfg.launches += 2;

@@ -100,46 +100,10 @@ __global__ void __launch_bounds__(256) grid_update_kernel(DMesh<D, T> M, GView<T
     }
 }
 
-// ---- sparse grid maintenance -------------------------------------------
+// ---- grid maintenance over the touched node blocks -----------------------
 // Node block B owns nodes [BW B, BW B + BW - 1] per axis. A particle block b
-// reaches nodes [BW b - 1, BW b + BW + 1], i.e. node blocks b-1 .. b+1 per axis.
-template <int D>
-__global__ void __launch_bounds__(128) mark_touched_kernel(const int* __restrict__ totals,
-                                                           const int* __restrict__ blocklist, int3 nb,
-                                                           unsigned char* __restrict__ cur) {
-    const int nactive = totals[0];
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nactive; i += gridDim.x * blockDim.x) {
-        const int b = blocklist[i] - 1;
-        const int bx = b % nb.x, by = (b / nb.x) % nb.y, bz = (D == 3) ? b / (nb.x * nb.y) : 0;
-        for (int dz = (D == 3 ? -1 : 0); dz <= (D == 3 ? 1 : 0); ++dz)
-            for (int dy = -1; dy <= 1; ++dy)
-                for (int dx = -1; dx <= 1; ++dx) {
-                    const int x = bx + dx, y = by + dy, z = bz + dz;
-                    if (x < 0 || y < 0 || z < 0 || x >= nb.x || y >= nb.y || (D == 3 && z >= nb.z)) continue;
-                    cur[x + nb.x * (y + nb.y * z)] = 1;
-                }
-    }
-}
-
-// The node blocks marked in cur or prev, compacted into a list (one atomic per
-// warp; the order of the list does not matter, every block is processed on its
-// own), so the zero and update passes visit the touched blocks only instead of
-// testing every block's flags.
-__global__ void __launch_bounds__(256) touched_list_kernel(const unsigned char* __restrict__ cur,
-                                                           const unsigned char* __restrict__ prev, int nblocks,
-                                                           int* __restrict__ list, int* __restrict__ count) {
-    const int lane = threadIdx.x & 31;
-    for (int B0 = blockIdx.x * blockDim.x; B0 < nblocks; B0 += gridDim.x * blockDim.x) {
-        const int B = B0 + threadIdx.x;
-        const bool t = B < nblocks && (cur[B] | prev[B]);
-        const unsigned m = __ballot_sync(0xffffffffu, t);
-        int base = 0;
-        if (lane == 0 && m) base = atomicAdd(count, __popc(m));
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (t) list[base + __popc(m & ((1u << lane) - 1u))] = B;
-    }
-}
-
+// reaches nodes [BW b - 1, BW b + BW + 1], i.e. node blocks b-1 .. b+1 per axis; the
+// scan of the binning lists the blocks reached now or in the previous transfer.
 // One warp per listed node block. mode 0: zero m, mv, f; mode 1: grid update
 // where cur, zero v, vn where the block was touched by the previous transfer only;
 // with zero_after, m, mv and f of the cur blocks are zeroed once read (the next
@@ -840,9 +804,6 @@ cudaError_t launch_g2p_kind(const DMesh<D, T>& M, const GView<T>& G, const PView
         else
             g2p_outside_kernel<D, T><<<og, 256, 0, cfg.stream>>>(P, s, b.blockids, b.totals);
     }
-    cudaError_t e = cudaSuccess;
-    if (count_next) e = cudaMemsetAsync(b.counts, 0, sizeof(int) * size_t(M.nblocks), cfg.stream);
-    if (e != cudaSuccess) return e;
     KernelScope ks(cfg, "g2p");
     kern<<<grid, 128, 0, cfg.stream>>>(M, G, P, s, b.totals, b.blocklist, b.offsets, b.perm, cfg.err,
                                        count_next ? b.blockids : nullptr, count_next ? b.counts : nullptr);
@@ -875,28 +836,6 @@ cudaError_t launch_g2p_direct(const DMesh<D, T>& M, const GView<T>& G, const PVi
         g2p_direct_kernel<D, T, D == 3><<<grid, 128, 0, cfg.stream>>>(M, G, P, s, cfg.err);
     else
         g2p_direct_kernel<D, T><<<grid, 128, 0, cfg.stream>>>(M, G, P, s, cfg.err);
-    ++*cfg.launches;
-    return cudaGetLastError();
-}
-
-cudaError_t launch_mark_touched(int dim, const int* nbv, const BinBuffers& b, unsigned char* cur, int nblocks,
-                                const LaunchCfg& cfg) {
-    const int grid = std::max(1, std::min((nblocks + 127) / 128, cfg.num_sms * 8));
-    const int3 nb = make_int3(nbv[0], nbv[1], nbv[2]);
-    KernelScope ks(cfg, "grid_mark");
-    if (dim == 3) mark_touched_kernel<3><<<grid, 128, 0, cfg.stream>>>(b.totals, b.blocklist, nb, cur);
-    else mark_touched_kernel<2><<<grid, 128, 0, cfg.stream>>>(b.totals, b.blocklist, nb, cur);
-    ++*cfg.launches;
-    return cudaGetLastError();
-}
-
-cudaError_t launch_touched_list(const unsigned char* cur, const unsigned char* prev, int nblocks, int* list,
-                                int* count, const LaunchCfg& cfg) {
-    cudaError_t e = cudaMemsetAsync(count, 0, sizeof(int), cfg.stream);
-    if (e != cudaSuccess) return e;
-    const int grid = std::max(1, std::min((nblocks + 255) / 256, cfg.num_sms * 8));
-    KernelScope ks(cfg, "grid_mark");
-    touched_list_kernel<<<grid, 256, 0, cfg.stream>>>(cur, prev, nblocks, list, count);
     ++*cfg.launches;
     return cudaGetLastError();
 }
