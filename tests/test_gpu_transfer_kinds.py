@@ -74,3 +74,37 @@ def test_one_step(tb, oracle, ctx, dim, ppc, sparse, basis, transfer, form):
         # weights there carry the rounding of the position relative to the support
         frac = np.mean(np.abs(got[k] - ref) > (tol if form == "f64" else 10 * tol) * scale)
         assert frac <= (0.0 if form == "f64" else 2e-3), (k, frac)
+
+
+@pytest.mark.parametrize("stretch", [1e-4, 0.02, 0.06, 0.2])
+@pytest.mark.parametrize("flow", [0.4e9, 1e13])
+def test_vonmises_strains(tb, oracle, ctx, stretch, flow):
+    """The von Mises update over elastic strains from the yield strain to far above
+    the range of its series (eigen-decomposition), plastic and elastic, FP64. The
+    tolerance is the Taylor tests' (1e-9)."""
+    from tesserae_b200 import runtime
+    abi = tb._abi
+    mesh = tb.CartesianMesh(0.1, (0.0, 1.0), (0.0, 1.0), (0.0, 1.0))
+    rng = np.random.default_rng(int(1e5 * stretch))
+    n = 3000
+    P = tb.Particles(n, 3, np.float64, optional=("eps_p", "Cp_inv"))
+    P.x[...] = rng.uniform(0.25, 0.75, size=(3, n))
+    P.v[...] = rng.normal(size=P.v.shape)
+    P.V[...] = 1e-3
+    A = stretch * rng.normal(size=(9, n)) / 3.0
+    P.F[...] += A
+    P.eps_p[...] = rng.uniform(0.0, 0.1, size=n)
+    mu, lam = tb.lame(117e9, 0.35)
+    prm = tb.step_params(1e-6, mass=1.0, V0=1e-3, mu=mu, lam=lam, basis=abi.TB_KC_BSPLINE_QUADRATIC,
+                         material=abi.MATERIAL_VONMISES, hardening=0.1e9, yield_stress=flow)
+    Pd = P.to("torch", device="cuda")
+    Po = P.to("numpy")
+    part = tb.Partition(mesh, n, backend="torch", device="cuda")
+    G = tb.generate_grid(mesh, np.float64, backend="torch", device="cuda")
+    runtime.step(G, Pd, part, mesh, prm, 1, ctx=ctx)
+    ctx.synchronize()
+    oracle.step(mesh, Po, tb.generate_grid(mesh, np.float64), prm, 1)
+    got = Pd.numpy()
+    for k in ("sigma", "Cp_inv", "eps_p", "V", "F"):
+        ref = getattr(Po, k)
+        assert np.abs(got[k] - ref).max() <= 1e-9 * np.abs(ref).max(), k
