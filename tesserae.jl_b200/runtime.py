@@ -46,6 +46,7 @@ class Context:
             stream = torch.cuda.current_stream(device)
         self.stream = stream
         handle = stream.cuda_stream if hasattr(stream, "cuda_stream") else int(stream or 0)
+        self.tape_held = 0  # device bytes of the tape buffers that this context keeps
         self.ptr = self.lib.tb_create(int(device), C.c_void_p(handle))
         if not self.ptr:
             raise RuntimeError("tb_create failed (no CUDA device?)")
@@ -89,6 +90,7 @@ class Context:
     def release_tape(self):
         """Free this context's tape buffers (the next tape_forward allocates again)."""
         self.check(self.lib.tb_tape_release(self.ptr), "tb_tape_release")
+        self.tape_held = 0
 
     def fn(self, name: str, dtype):
         return getattr(self.lib, f"{name}_{_suffix(dtype)}")
@@ -303,12 +305,18 @@ def tape_slot_bytes(mesh: CartesianMesh, n: int, dtype, apic: bool = False, x64:
 
 
 def choose_checkpoint_every(mesh: CartesianMesh, n: int, dtype, nsteps: int, apic: bool = False,
-                            device=None, budget: float = 0.6, fallback: int = 20, x64: bool = False) -> int:
+                            device=None, budget: float = 0.6, fallback: int = 20, x64: bool = False,
+                            ctx: Context | None = None) -> int:
     """1 (the whole tape in device memory) when it takes at most `budget` of the
-    device's free memory, else `fallback`."""
+    device's free memory, else `fallback`. A tape that fits in the buffers `ctx`
+    already keeps needs no more memory: the driver's free-memory query, a good part
+    of a millisecond, is left out then."""
     import torch
+    need = tape_bytes(mesh, n, dtype, nsteps, 1, apic, x64)
+    if ctx is not None and need <= ctx.tape_held:
+        return 1
     free, _ = torch.cuda.mem_get_info(device)
-    return 1 if tape_bytes(mesh, n, dtype, nsteps, 1, apic, x64) <= budget * free else fallback
+    return 1 if need <= budget * free else fallback
 
 
 def tape_forward(grid: Grid, particles: Particles, partition: Partition, mesh: CartesianMesh, params,
@@ -317,10 +325,16 @@ def tape_forward(grid: Grid, particles: Particles, partition: Partition, mesh: C
     `checkpoint_every` steps; 1 keeps every step's state, grid and partition (the
     whole tape), so tape_backward runs no forward step."""
     ctx = ctx or _default()
+    held, ctx.tape_held = ctx.tape_held, 0  # a failed allocation leaves no buffer
     rc = ctx.pfn("tb_tape_forward", particles, x64_ok=True)(ctx.ptr, _ref(mesh.struct()), _ref(particles.struct()),
                                                     _ref(partition.struct()), _ref(grid.struct()), _ref(params),
                                                     int(nsteps), int(checkpoint_every))
     ctx.check(rc, "tape_forward")
+    ctx.tape_held = held
+    if int(checkpoint_every) == 1:
+        ctx.tape_held = max(held, tape_bytes(mesh, particles.n, particles.dtype, nsteps, 1,
+                                             params.transfer == _abi.TB_TRANSFER_APIC,
+                                             getattr(particles, "x64", False)))
 
 
 def tape_backward(grid: Grid, particles: Particles, partition: Partition, mesh: CartesianMesh, params,
@@ -352,7 +366,7 @@ def rollout_grad(particles: Particles, mesh: CartesianMesh, params, nsteps: int,
     if checkpoint_every is None:
         checkpoint_every = choose_checkpoint_every(mesh, n, particles.dtype, nsteps,
                                                    params.transfer == _abi.TB_TRANSFER_APIC, particles.device,
-                                                   x64=getattr(particles, "x64", False))
+                                                   x64=getattr(particles, "x64", False), ctx=ctx)
     part = Partition(mesh, n, backend="torch", device=particles.device or "cuda")
     grid = Grid(mesh, particles.dtype, backend="torch", device=particles.device or "cuda")
     tape_forward(grid, particles, part, mesh, params, nsteps, checkpoint_every, ctx=ctx)
@@ -382,7 +396,7 @@ class RolloutFunction:
         if checkpoint_every is None:
             checkpoint_every = choose_checkpoint_every(mesh, particles.n, particles.dtype, nsteps,
                                                        params.transfer == _abi.TB_TRANSFER_APIC, v0.device,
-                                                       x64=getattr(particles, "x64", False))
+                                                       x64=getattr(particles, "x64", False), ctx=ctx or _default())
 
         class _F(torch.autograd.Function):
             @staticmethod

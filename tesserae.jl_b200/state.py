@@ -31,12 +31,15 @@ def _ptr(a) -> int | None:
 
 
 def _row_ptrs(a, k: int) -> list[int | None]:
-    """Pointers to rows 0..k-1 of a (k, n) array."""
+    """Pointers to rows 0..k-1 of a (k, n) array, from its base and row stride (a
+    view object per row cost about 1 us each, 40 of them on every call)."""
     if a is None:
         return [None] * k
     if isinstance(a, np.ndarray):
-        return [a[i].ctypes.data for i in range(k)]
-    return [a[i].data_ptr() for i in range(k)]
+        base, step = a.ctypes.data, a.strides[0]
+    else:
+        base, step = a.data_ptr(), a.stride(0) * a.element_size()
+    return [base + i * step for i in range(k)]
 
 
 # ---------------------------------------------------------------------------
@@ -189,27 +192,20 @@ class Particles:
         s = _abi.tb_particles()
         D = self.dim
         s.n = self.n
-        for d, p in enumerate(_row_ptrs(self.x, D)):
-            s.x[d] = p
-        for d, p in enumerate(_row_ptrs(self.v, D)):
-            s.v[d] = p
+        s.x[:D] = _row_ptrs(self.x, D)
+        s.v[:D] = _row_ptrs(self.v, D)
         s.V = _ptr(self.V)
         s.m = _ptr(self.m)
         s.l = _ptr(self.l)
-        for k, p in enumerate(_row_ptrs(self.grad_v, D * D)):
-            s.grad_v[k] = p
-        for k, p in enumerate(_row_ptrs(self.sigma, nsym(D))):
-            s.sigma[k] = p
-        for k, p in enumerate(_row_ptrs(self.F, D * D)):
-            s.F[k] = p
-        for k, p in enumerate(_row_ptrs(self.B, D * D)):
-            s.B[k] = p
+        s.grad_v[:D * D] = _row_ptrs(self.grad_v, D * D)
+        s.sigma[:nsym(D)] = _row_ptrs(self.sigma, nsym(D))
+        s.F[:D * D] = _row_ptrs(self.F, D * D)
+        s.B[:D * D] = _row_ptrs(self.B, D * D)
         s.V0 = _ptr(self.V0)
         s.mu = _ptr(self.mu)
         s.lambda_ = _ptr(self.lam)
         s.eps_p = _ptr(self.eps_p)
-        for k, p in enumerate(_row_ptrs(self.Cp_inv, nsym(D))):
-            s.Cp_inv[k] = p
+        s.Cp_inv[:nsym(D)] = _row_ptrs(self.Cp_inv, nsym(D))
         return s
 
     def to(self, backend, device=None, dtype=None, x64=None) -> "Particles":
@@ -273,16 +269,12 @@ class Adjoint:
     def struct(self) -> _abi.tb_adjoint:
         s = _abi.tb_adjoint()
         D = self.dim
-        for d, p in enumerate(_row_ptrs(self.x, D)):
-            s.x[d] = p
-        for d, p in enumerate(_row_ptrs(self.v, D)):
-            s.v[d] = p
-        for k, p in enumerate(_row_ptrs(self.F, D * D)):
-            s.F[k] = p
+        s.x[:D] = _row_ptrs(self.x, D)
+        s.v[:D] = _row_ptrs(self.v, D)
+        s.F[:D * D] = _row_ptrs(self.F, D * D)
         s.mu = _ptr(self.mu)
         s.lambda_ = _ptr(self.lam)
-        for k, p in enumerate(_row_ptrs(self.B, D * D)):
-            s.B[k] = p
+        s.B[:D * D] = _row_ptrs(self.B, D * D)
         return s
 
     def numpy(self) -> dict:
@@ -352,9 +344,7 @@ class Grid:
         D = self.mesh.dim
         s.m = _ptr(self.m)
         for name in ("mv", "f", "v", "vn"):
-            arr = getattr(s, name)
-            for d, p in enumerate(_row_ptrs(getattr(self, name), D)):
-                arr[d] = p
+            getattr(s, name)[:D] = _row_ptrs(getattr(self, name), D)
         if self.sparse:
             s.block_numbering = _ptr(self.block_numbering)
             s.active_blocks = _ptr(self.active_blocks)
