@@ -258,8 +258,11 @@ __global__ void __launch_bounds__(128, g2p_ctas(GEN, VM, sizeof(T) == 4)) g2p_ti
     const int nactive = totals[0];
     const int tid = threadIdx.x, nth = blockDim.x;
     // CTA `piece` of `split` sharing a block takes its particles piece nth + tid,
-    // (piece + split) nth + tid, ... (block_split: 4 particles per thread)
-    const int split = block_split(totals, 4 * nth);
+    // (piece + split) nth + tid, ... (4 particles per thread; fewer, down to one, where
+    // the blocks are fewer than the CTAs: a 111 k particle 2D scene of 200 blocks,
+    // 0.0209 -> 0.0148 ms per step)
+    int per;
+    const int split = max(block_split(totals, 4 * nth), block_pieces(totals, nactive, 4 * nth, gridDim.x, per));
     const int stride = split * nth;
     for (int vi = blockIdx.x; vi < nactive * split; vi += gridDim.x) {
         const int bi = split == 1 ? vi : vi / split, piece = vi - bi * split;
