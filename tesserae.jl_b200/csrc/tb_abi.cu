@@ -329,7 +329,10 @@ int bin_buffers(tb_ctx* c, const tb_partition* part, long long n, long long nb, 
     return TB_OK;
 }
 
-LaunchCfg cfg_of(tb_ctx* c) { return LaunchCfg{c->stream, c->num_sms, &c->launches, c->d_err, c->prof}; }
+// `n`: the particles of the call's kernels (launches are set up early on small scenes).
+LaunchCfg cfg_of(tb_ctx* c, long long n = EARLY_N + 1) {
+    return LaunchCfg{c->stream, c->num_sms, &c->launches, c->d_err, c->prof, n <= EARLY_N};
+}
 
 // Reads and clears the device status word (synchronises the stream).
 int check_device_status(tb_ctx* c) {
@@ -507,7 +510,7 @@ int run_step(tb_ctx* c, const tb_mesh* m, tb_particles* p, tb_partition* part, t
     if ((rc = make_gview<T>(c, g, D, G, m->block_log2)) != TB_OK) return rc;
     BinBuffers B;
     if ((rc = bin_buffers(c, part, P.n, M.nblocks, B)) != TB_OK) return rc;
-    const LaunchCfg cfg = cfg_of(c);
+    const LaunchCfg cfg = cfg_of(c, P.n);
     const T* xs[3] = {P.x[0], P.x[1], D == 3 ? P.x[2] : P.x[1]};
     // FP64 positions are binned by the FP64 findblock (the reference's Float64 rule)
     const auto M64 = make_dmesh<D, double>(*m);
@@ -630,7 +633,7 @@ int do_bin_only(tb_ctx* c, const tb_mesh* m, const tb_particles* p, tb_partition
     if ((rc = make_pview<T>(c, p, m->dim, false, false, P)) != TB_OK) return rc;
     BinBuffers B;
     if ((rc = bin_buffers(c, part, P.n, mesh_nblocks(m), B)) != TB_OK) return rc;
-    const LaunchCfg cfg = cfg_of(c);
+    const LaunchCfg cfg = cfg_of(c, P.n);
     const T* xs[3] = {P.x[0], P.x[1], m->dim == 3 ? P.x[2] : P.x[1]};
     cudaError_t e = (m->dim == 3) ? launch_bin<3, T>(make_dmesh<3, T>(*m), xs, P.n, B, cfg)
                                   : launch_bin<2, T>(make_dmesh<2, T>(*m), xs, P.n, B, cfg);

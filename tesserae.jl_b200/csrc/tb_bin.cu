@@ -32,6 +32,7 @@ __global__ void __launch_bounds__(256) bin_count_kernel(DMesh<D, T> M, const T* 
                                                         const T* __restrict__ x1, const T* __restrict__ x2,
                                                         long long n, int* __restrict__ blockids,
                                                         int* __restrict__ counts) {
+    chain_wait();
     const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     int b = -1;
     if (p < n) {
@@ -80,6 +81,7 @@ __device__ __forceinline__ unsigned long long block_incl_scan(unsigned long long
 
 __global__ void __launch_bounds__(256) scan_reduce_kernel(const int* __restrict__ counts, int nb,
                                                           unsigned long long* __restrict__ partials) {
+    chain_wait();
     __shared__ unsigned long long wt[8];
     const int base = blockIdx.x * SCAN_TILE + threadIdx.x * 4;
     unsigned long long s = 0;
@@ -107,6 +109,7 @@ __global__ void __launch_bounds__(256) scan_kernel(const int* __restrict__ count
                                                    int* __restrict__ offsets, int* __restrict__ cursors,
                                                    int* __restrict__ blocklist, int* __restrict__ totals,
                                                    unsigned long long* __restrict__ bnd_count, TouchArgs touch) {
+    chain_wait();
     __shared__ unsigned long long wt[8];
     const int tile0 = blockIdx.x * SCAN_TILE, base = tile0 + threadIdx.x * 4;
     unsigned long long before = 0;
@@ -181,6 +184,7 @@ __global__ void __launch_bounds__(256) scan_kernel(const int* __restrict__ count
 constexpr int SCAT_IT = 4;
 __global__ void __launch_bounds__(256) bin_scatter_kernel(const int* __restrict__ blockids, long long n,
                                                           int* __restrict__ cursors, int* __restrict__ perm_tmp) {
+    chain_wait();
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const long long c0 = (((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (32ll * SCAT_IT);
@@ -493,6 +497,7 @@ __global__ void __launch_bounds__(FIX_THREADS) bin_fixup_kernel(const int* __res
                                                                 const int* __restrict__ S, int* __restrict__ perm,
                                                                 unsigned long long* __restrict__ gscratch,
                                                                 int* __restrict__ zero, int nb) {
+    chain_wait();
     constexpr int NWARP = FIX_THREADS / 32;
     __shared__ FixShared sm;
     __shared__ int whpos[NWARP][FIXW_RUNS + 1], whkey[NWARP][FIXW_RUNS], whout[NWARP][FIXW_RUNS];
@@ -527,13 +532,13 @@ void launch_scan(const int* counts, int nb, unsigned long long* partials, int* o
                  int* totals, unsigned long long* bnd_count, const TouchArgs& touch, const LaunchCfg& cfg) {
     const int nt = scan_tiles(nb);
     if (nt <= SCAN_ONE) {
-        scan_kernel<true><<<nt, 256, 0, cfg.stream>>>(counts, nb, partials, offsets, cursors, blocklist, totals,
+        launch_chained(scan_kernel<true>, nt, 256, 0, cfg, counts, nb, partials, offsets, cursors, blocklist, totals,
                                                       bnd_count, touch);
         ++*cfg.launches;
         return;
     }
-    scan_reduce_kernel<<<nt, 256, 0, cfg.stream>>>(counts, nb, partials);
-    scan_kernel<false><<<nt, 256, 0, cfg.stream>>>(counts, nb, partials, offsets, cursors, blocklist, totals, bnd_count,
+    launch_chained(scan_reduce_kernel, nt, 256, 0, cfg, counts, nb, partials);
+    launch_chained(scan_kernel<false>, nt, 256, 0, cfg, counts, nb, partials, offsets, cursors, blocklist, totals, bnd_count,
                                                    touch);
     *cfg.launches += 2;
 }
@@ -596,7 +601,7 @@ cudaError_t launch_bin_count(const DMesh<D, T>& M, const T* const* x, long long 
     if (e != cudaSuccess) return e;
     if (n > 0) {
         KernelScope ks(cfg, "bin_count");
-        bin_count_kernel<D, T><<<grid_for(n, 256), 256, 0, cfg.stream>>>(M, x[0], x[1], D == 3 ? x[2] : x[1], n,
+        launch_chained(bin_count_kernel<D, T>, grid_for(n, 256), 256, 0, cfg, M, x[0], x[1], D == 3 ? x[2] : x[1], n,
                                                                          b.blockids, b.counts);
         ++*cfg.launches;
     }
@@ -612,12 +617,12 @@ cudaError_t launch_bin_rest(int nb, long long n, const BinBuffers& b, const Laun
     if (n > 0) {
         {
             KernelScope ks(cfg, "bin_scatter");
-            bin_scatter_kernel<<<grid_for(n, 256 * SCAT_IT), 256, 0, cfg.stream>>>(b.blockids, n, b.cursors,
+            launch_chained(bin_scatter_kernel, grid_for(n, 256 * SCAT_IT), 256, 0, cfg, b.blockids, n, b.cursors,
                                                                                   b.perm_tmp);
         }
         KernelScope ks(cfg, "bin_fixup");
         const int grid = std::max(1, std::min(nb, cfg.num_sms * 5));
-        bin_fixup_kernel<<<grid, FIX_THREADS, 0, cfg.stream>>>(b.totals, b.blocklist, b.offsets, b.perm_tmp, b.perm,
+        launch_chained(bin_fixup_kernel, grid, FIX_THREADS, 0, cfg, b.totals, b.blocklist, b.offsets, b.perm_tmp, b.perm,
                                                                b.sort_scratch, zero_counts ? b.counts : nullptr, nb);
         *cfg.launches += 2;
     }

@@ -370,6 +370,7 @@ __global__ void __launch_bounds__(P2G_THREADS, CTAS)
                       const int* __restrict__ blocklist, const int* __restrict__ offsets,
                       const int* __restrict__ perm, int* err, const int* __restrict__ list,
                       const unsigned long long* __restrict__ nlist) {
+    chain_wait();
     using SH = PencilShape<3, 4>;
     using T2 = typename PairOf<T>::type;
     constexpr int NT = P2G_THREADS, NW = NT / 32, ITEMS = (NR + NT - 1) / NT, RS = RecOf<KIND>::SIZE;
@@ -602,7 +603,7 @@ cudaError_t launch_pencil(const DMesh<3, T>& M, const PView<T>& P, const GView<T
     int grid = 0;
     cudaError_t e = prepare_launch(kern, P2G_THREADS, smem, cfg, M.nblocks, grid);
     if (e != cudaSuccess) return e;
-    kern<<<grid, P2G_THREADS, smem, cfg.stream>>>(M, P, G, s, b.totals, b.blocklist, b.offsets, b.perm, cfg.err, list,
+    launch_chained(kern, grid, P2G_THREADS, smem, cfg, M, P, G, s, b.totals, b.blocklist, b.offsets, b.perm, cfg.err, list,
                                                  nlist);
     ++*cfg.launches;
     return cudaGetLastError();
@@ -694,6 +695,7 @@ __global__ void __launch_bounds__(PLANE_THREADS, 3)
                      const int* __restrict__ totals, const int* __restrict__ blocklist,
                      const int* __restrict__ offsets, const int* __restrict__ perm, int* err,
                      int* __restrict__ bnd, unsigned long long* __restrict__ bnd_count) {
+    chain_wait();
     using SH = PencilShape<3, 4>;
     constexpr int NT = PLANE_THREADS, NR = PLANE_NR, ITEMS = NR / NT;
     constexpr int TS = SH::TS, TN = SH::TN, NC = SH::NC, G1 = SH::G1, NG = SH::NG;
@@ -948,7 +950,7 @@ cudaError_t launch_plane(const DMesh<3, float>& M, const PView<float>& P, const 
     int grid = 0;
     cudaError_t e = prepare_launch(kern, PLANE_THREADS, smem, cfg, M.nblocks, grid);
     if (e != cudaSuccess) return e;
-    kern<<<grid, PLANE_THREADS, smem, cfg.stream>>>(M, P, G, s, b.totals, b.blocklist, b.offsets, b.perm, cfg.err,
+    launch_chained(kern, grid, PLANE_THREADS, smem, cfg, M, P, G, s, b.totals, b.blocklist, b.offsets, b.perm, cfg.err,
                                                    bnd, bnd_count);
     ++*cfg.launches;
     return cudaGetLastError();
@@ -990,6 +992,7 @@ __global__ void __launch_bounds__(P2D_THREADS, 4)
     p2g_2d_kernel(DMesh<2, T> M, PView<T> P, GView<T> G, Scalars<T> s, const int* __restrict__ totals,
                   const int* __restrict__ blocklist, const int* __restrict__ offsets, const int* __restrict__ perm,
                   int* err) {
+    chain_wait();
     using SH = PencilShape<2, BW>;
     using R = Rec2<KIND>;
     using T2 = typename PairOf<T>::type;
@@ -1275,7 +1278,7 @@ cudaError_t launch_2d_kind(const DMesh<2, T>& M, const PView<T>& P, const GView<
     int grid = 0;
     cudaError_t e = prepare_launch(kern, P2D_THREADS, smem, cfg, M.nblocks, grid);
     if (e != cudaSuccess) return e;
-    kern<<<grid, P2D_THREADS, smem, cfg.stream>>>(M, P, G, s, b.totals, b.blocklist, b.offsets, b.perm, cfg.err);
+    launch_chained(kern, grid, P2D_THREADS, smem, cfg, M, P, G, s, b.totals, b.blocklist, b.offsets, b.perm, cfg.err);
     ++*cfg.launches;
     return cudaGetLastError();
 }

@@ -37,6 +37,7 @@ __device__ __forceinline__ long long stored_nodes(const GView<T>& G, long long n
 
 template <int D, class T>
 __global__ void __launch_bounds__(256) grid_zero_kernel(GView<T> G, long long nnodes) {
+    chain_wait();
     const long long nn = stored_nodes<D>(G, nnodes);
     for (long long I = (long long)blockIdx.x * blockDim.x + threadIdx.x; I < nn; I += (long long)gridDim.x * blockDim.x) {
         G.m[I] = T(0);
@@ -77,6 +78,7 @@ __device__ __forceinline__ void update_node(const DMesh<D, T>& M, const GView<T>
 // untouched blocks gained nothing: the pass is bound by its six stores per node.
 template <int D, class T>
 __global__ void __launch_bounds__(256) grid_update_kernel(DMesh<D, T> M, GView<T> G, Scalars<T> s) {
+    chain_wait();
     const int lane = threadIdx.x & 31;
     const int nrows = D == 3 ? M.n[1] * M.n[2] : M.n[1], warps = (gridDim.x * blockDim.x) >> 5;
     for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < nrows; r += warps) {
@@ -129,6 +131,7 @@ __global__ void __launch_bounds__(256) node_list_kernel(DMesh<D, T> M, GView<T> 
                                                         const unsigned char* __restrict__ cur,
                                                         const int* __restrict__ list, const int* __restrict__ count,
                                                         int zero_after) {
+    chain_wait();
     constexpr int NPB = (D == 3) ? BW * BW * BW : BW * BW;
     const int lane = threadIdx.x & 31;
     const int warps = (gridDim.x * blockDim.x) >> 5;
@@ -229,6 +232,7 @@ __global__ void __launch_bounds__(128, g2p_ctas(GEN, VM, sizeof(T) == 4)) g2p_ti
                                                        const int* __restrict__ offsets,
                                                        const int* __restrict__ perm, int* err,
                                                        int* __restrict__ next_bid, int* __restrict__ next_count) {
+    chain_wait();
     constexpr int TS = Tile<D, BW>::TS, TN = Tile<D, BW>::TN;
     constexpr bool WLS = GEN == G_WLS || GEN == G_WLS_APIC, APIC = GEN == G_WLS_APIC || GEN == G_APIC;
     // 3D FP32: node-major, (v_x, v_y, v_z, dv_x) as a float4 at [t] and (dv_y, dv_z)
@@ -723,6 +727,7 @@ __global__ void __launch_bounds__(128) g2p_direct_kernel(DMesh<D, T> M, GView<T>
 template <int D, class T, bool VM = false>
 __global__ void __launch_bounds__(256) g2p_outside_kernel(PView<T> P, Scalars<T> s, const int* __restrict__ blockids,
                                                           const int* __restrict__ totals) {
+    chain_wait();
     if ((long long)totals[1] >= P.n) return;  // every particle is inside a block
     for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < P.n; p += (long long)gridDim.x * blockDim.x) {
         if (blockids[p] != 0) continue;
@@ -825,7 +830,7 @@ cudaError_t launch_grid_zero(const DMesh<D, T>& M, const GView<T>& G, const Laun
         return cudaSuccess;
     }
     const int grid = int(std::min<long long>((nn + 255) / 256, (long long)cfg.num_sms * 16));
-    grid_zero_kernel<D, T><<<grid, 256, 0, cfg.stream>>>(G, nn);
+    launch_chained(grid_zero_kernel<D, T>, grid, 256, 0, cfg, G, nn);
     ++*cfg.launches;
     return cudaGetLastError();
 }
@@ -839,7 +844,7 @@ cudaError_t launch_grid_update(const DMesh<D, T>& M, const GView<T>& G, const Sc
     } else {
         const long long rows = D == 3 ? (long long)M.n[1] * M.n[2] : M.n[1];
         const int grid = int(std::min<long long>((rows + 7) / 8, (long long)cfg.num_sms * 16));
-        grid_update_kernel<D, T><<<grid, 256, 0, cfg.stream>>>(M, G, s);
+        launch_chained(grid_update_kernel<D, T>, grid, 256, 0, cfg, M, G, s);
     }
     ++*cfg.launches;
     return cudaGetLastError();
@@ -867,13 +872,13 @@ cudaError_t launch_g2p_kind(const DMesh<D, T>& M, const GView<T>& G, const PView
         KernelScope ks(cfg, "g2p_outside");
         const int og = int(std::min<long long>((P.n + 255) / 256, (long long)cfg.num_sms * 8));
         if (D == 3 && s.material == TB_MATERIAL_VONMISES)
-            g2p_outside_kernel<D, T, D == 3><<<og, 256, 0, cfg.stream>>>(P, s, b.blockids, b.totals);
+            launch_chained(g2p_outside_kernel<D, T, D == 3>, og, 256, 0, cfg, P, s, b.blockids, b.totals);
         else
-            g2p_outside_kernel<D, T><<<og, 256, 0, cfg.stream>>>(P, s, b.blockids, b.totals);
+            launch_chained(g2p_outside_kernel<D, T>, og, 256, 0, cfg, P, s, b.blockids, b.totals);
     }
     KernelScope ks(cfg, "g2p");
-    kern<<<grid, 128, 0, cfg.stream>>>(M, G, P, s, b.totals, b.blocklist, b.offsets, b.perm, cfg.err,
-                                       count_next ? b.blockids : nullptr, count_next ? b.counts : nullptr);
+    launch_chained(kern, grid, 128, 0, cfg, M, G, P, s, b.totals, b.blocklist, b.offsets, b.perm, cfg.err,
+                   count_next ? b.blockids : nullptr, count_next ? b.counts : nullptr);
     *cfg.launches += 2;
     return cudaGetLastError();
 }
@@ -923,7 +928,7 @@ cudaError_t launch_sparse_zero(const DMesh<D, T>& M, const GView<T>& G, const in
                                const LaunchCfg& cfg) {
     const int grid = int(std::max(1ll, std::min((M.nblocks * 32ll + 255) / 256, cfg.num_sms * 16ll)));
     KernelScope ks(cfg, "grid_zero");
-    node_list_kernel<D, T, BW, 0><<<grid, 256, 0, cfg.stream>>>(M, G, Scalars<T>{}, nullptr, list, count, 0);
+    launch_chained(node_list_kernel<D, T, BW, 0>, grid, 256, 0, cfg, M, G, Scalars<T>{}, nullptr, list, count, 0);
     ++*cfg.launches;
     return cudaGetLastError();
 }
@@ -934,7 +939,7 @@ cudaError_t launch_sparse_grid_update(const DMesh<D, T>& M, const GView<T>& G, c
                                       const LaunchCfg& cfg, bool zero_after) {
     const int grid = int(std::max(1ll, std::min((M.nblocks * 32ll + 255) / 256, cfg.num_sms * 16ll)));
     KernelScope ks(cfg, "grid_update");
-    node_list_kernel<D, T, BW, 1><<<grid, 256, 0, cfg.stream>>>(M, G, s, cur, list, count, zero_after ? 1 : 0);
+    launch_chained(node_list_kernel<D, T, BW, 1>, grid, 256, 0, cfg, M, G, s, cur, list, count, zero_after ? 1 : 0);
     ++*cfg.launches;
     return cudaGetLastError();
 }
