@@ -214,7 +214,7 @@ __device__ __forceinline__ void g2p_finish(const PView<T>& P, const Scalars<T>& 
 //   G_APIC     plain kernel, APIC: the contraction with the first moments of r
 // Before the closed form every WLS / APIC particle evaluated a (D+1)^2 moment
 // inverse at each of its nodes: dam break at half resolution, 18.2 M particles,
-// FP32 with FP64 positions, 3.66 ms; 1.83 ms now.
+// FP32 with FP64 positions, 3.66 ms; 1.75 ms now.
 enum : int { G_PLAIN = 0, G_WLS = 1, G_WLS_APIC = 2, G_APIC = 3 };
 
 // CTAs of 128 threads per SM. General kinds in FP32: 6 (80 registers) measured 1.92
@@ -351,41 +351,56 @@ __global__ void __launch_bounds__(128, g2p_ctas(GEN, VM, sizeof(T) == 4)) g2p_ti
                 if (!ok) {
                     atomicOr(err, ERR_TILE_RANGE);
                 } else if (WLS && B.cut) {
-                    // a WLS window that the mesh cuts: per-node weights
+                    // A WLS window that the mesh cuts, row by row: N_x = wx R + gx Q with
+                    // R = wyz - u_y dyz - u_z wdz, Q = -u_x wyz. The row loops are not
+                    // unrolled (jets by selection): few particles come here, and 27
+                    // unrolled nodes made the kernel wait for instructions (dam break:
+                    // 1.83 ms against 1.75).
+                    auto sel = [](const T* q, int k) { return k == 0 ? q[0] : (k == 1 ? q[1] : q[2]); };
+                    auto rel = [&](int d, int k) {
+                        if constexpr (X64)  // X_i - x_p in FP64, rounded once
+                            return T(__dadd_rn(M.xmin64[d], __dmul_rn(double(B.ax[d].lo + k), M.h64)) - xd[d]);
+                        else
+                            return node_coord(M, d, B.ax[d].lo + k) - x[d];
+                    };
+#pragma unroll 1
+                    for (int jk = 0; jk < (D == 3 ? 9 : 3); ++jk) {
+                        const int k = jk / 3, jj = jk - 3 * k;
+                        const T wy = sel(B.ax[1].val, jj), gy = sel(B.ax[1].der, jj) * M.h_inv;
+                        T wz = T(1), gz = T(0);
+                        if constexpr (D == 3) {
+                            wz = sel(B.ax[D - 1].val, k);
+                            gz = sel(B.ax[D - 1].der, k) * M.h_inv;
+                        }
+                        const T wyz = wy * wz, dyz = gy * wz, wdz = wy * gz;
+                        T R = wyz - B.u[1] * dyz;
+                        if constexpr (D == 3) R -= B.u[D - 1] * wdz;
+                        const T Q = -B.u[0] * wyz;
+                        const T ry = APIC ? rel(1, jj) : T(0), rz = (APIC && D == 3) ? rel(D - 1, k) : T(0);
+                        const int t0 = (D == 3) ? q0[0] + TS * ((q0[1] + jj) + TS * (q0[D - 1] + k))
+                                                : q0[0] + TS * (q0[1] + jj);
 #pragma unroll
-                    for (int k = 0; k < (D == 3 ? 3 : 1); ++k)
+                        for (int i = 0; i < 3; ++i) {
+                            const T wx = B.ax[0].val[i], gx = B.ax[0].der[i] * M.h_inv, N = wx * R + gx * Q;
+                            T vi[3], dvi[3];
+                            node_vals(t0 + i, vi, dvi);
+                            const T rx = APIC ? rel(0, i) : T(0);
 #pragma unroll
-                        for (int jj = 0; jj < 3; ++jj)
-#pragma unroll
-                            for (int i = 0; i < 3; ++i) {
-                                const int idx[3] = {i, jj, k};
-                                const int t = (D == 3) ? (q0[0] + i) + TS * ((q0[1] + jj) + TS * (q0[D - 1] + k))
-                                                       : (q0[0] + i) + TS * (q0[1] + jj);
-                                T w, dw[3];
-                                eval_node<D, T>(M, B, i, jj, k, w, dw);
-                                T vi[3], dvi[3];
-                                node_vals(t, vi, dvi);
-#pragma unroll
-                                for (int r = 0; r < D; ++r) {
-                                    vpic[r] += w * vi[r];
-                                    if constexpr (!APIC) dvf[r] += w * dvi[r];
-#pragma unroll
-                                    for (int c = 0; c < D; ++c) gv[r][c] += vi[r] * dw[c];
-                                }
+                            for (int r = 0; r < D; ++r) {
+                                const T Nv = N * vi[r];
+                                vpic[r] += Nv;
+                                if constexpr (!APIC) dvf[r] += N * dvi[r];
+                                gv[r][0] += (gx * wyz) * vi[r];
+                                gv[r][1] += (wx * dyz) * vi[r];
+                                if constexpr (D == 3) gv[r][2] += (wx * wdz) * vi[r];
                                 if constexpr (APIC) {
-#pragma unroll
-                                    for (int c = 0; c < D; ++c) {
-                                        T rel;
-                                        if constexpr (X64)  // X_i - x_p in FP64, rounded once
-                                            rel = T(__dadd_rn(M.xmin64[c], __dmul_rn(double(B.ax[c].lo + idx[c]), M.h64)) -
-                                                    xd[c]);
-                                        else
-                                            rel = node_coord(M, c, B.ax[c].lo + idx[c]) - x[c];
-#pragma unroll
-                                        for (int r = 0; r < D; ++r) Bn[r][c] += (w * vi[r]) * rel;
-                                    }
+                                    Bn[r][0] += Nv * rx;
+                                    Bn[r][1] += Nv * ry;
+                                    if constexpr (D == 3) Bn[r][2] += Nv * rz;
                                 }
                             }
+                        }
+                    }
                 } else if constexpr (APIC && VEC) {
                     float gx[3], rr[3][3];
 #pragma unroll
