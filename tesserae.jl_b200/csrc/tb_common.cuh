@@ -45,8 +45,9 @@ __device__ __forceinline__ int block_split(const int* totals, int per_cta) {
 
 // CTAs that share one block in a kernel that takes passes of up to `nb` particles
 // and may sum several passes before it adds them to the grid, for `nblk` blocks
-// on a grid of `ctas`: enough for about four pieces per CTA while every piece
-// still has a full pass, and for one piece per CTA where the blocks are fewer than
+// on a grid of `ctas`: enough for about twelve pieces per CTA while every piece
+// still has a full pass (2.1 M-particle FP64 sphere of 64 per cell: P2G 0.455 ms at four,
+// 0.378 at twelve), and for one piece per CTA where the blocks are fewer than
 // the CTAs (passes of `per` < nb particles then, at least 128). Short passes cost:
 // a 64^3 B-spline block of 262 k particles (512 blocks on 444 CTAs) took 5% longer
 // per step with two half passes per block than with one.
@@ -55,7 +56,7 @@ __device__ __forceinline__ int block_pieces(const int* totals, int nblk, int nb,
     const int nact = totals[0];
     if (nact <= 0 || nblk <= 0) return 1;
     const int avg = int((long long)totals[1] / nact), passes = (avg + nb - 1) / nb;
-    const int full = min(passes, (4 * ctas + nblk - 1) / nblk), fill = min(ctas / nblk, (avg + 127) / 128);
+    const int full = min(passes, (12 * ctas + nblk - 1) / nblk), fill = min(ctas / nblk, (avg + 127) / 128);
     const int pieces = max(1, min(8, max(full, fill)));
     if (pieces > passes) per = min(nb, max(128, ((avg + pieces - 1) / pieces + 7) & ~7));
     return pieces;
@@ -652,6 +653,12 @@ __device__ __forceinline__ bool prepare_basis(const DMesh<D, T>& M, int basis, c
     }
     B.wls = ALLOW_WLS && (basis == TB_WLS_BSPLINE_QUADRATIC || basis == TB_WLS_UGIMP);
     if constexpr (ALLOW_WLS) if (B.wls) {
+        if constexpr (sizeof(T) == 4) {
+            // FP32 positions: node coordinates rounded one by one leave sum w and
+            // sum w r off by 1e-5, which the moments put right on every window (left
+            // out, the dam break's 100-step error in v was 3e-5 instead of 1e-6)
+            if (basis == TB_WLS_UGIMP) B.cut = cut[0] = cut[1] = cut[2] = true;
+        }
         T r[3][3] = {};
 #pragma unroll
         for (int d = 0; d < D; ++d)
