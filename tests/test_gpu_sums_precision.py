@@ -1,4 +1,5 @@
-"""Bits that the FP32 transfers keep in the sums of a crowded block."""
+"""Bits that the transfers keep: sums of a crowded block, and the consistency of WLS
+weights far from the origin."""
 import numpy as np
 import pytest
 
@@ -51,3 +52,35 @@ def test_crowded_block_2d_sums_in_fp64(tb, ctx, transfer, basis):
     for d, v in enumerate((1.0, -0.5)):
         gv = got["mv"][d].astype(np.float64).reshape(m.shape)
         assert np.max(np.abs(gv - v * m)[on] / m[on]) <= tol
+
+
+@pytest.mark.parametrize("basis", ["wls_bspline_quadratic", "wls_ugimp"])
+@pytest.mark.parametrize("dim", [2, 3])
+def test_wls_weights_reproduce_constants_far_from_the_origin(tb, ctx, dim, basis):
+    """FP32: sum N = 1 and sum grad N = 0 wherever WLS fits its moments (uGIMP; B-spline
+    windows that the mesh cuts), although a node's coordinate is rounded by up to
+    eps |X| (|X| / h = 1300 here, so a weight is off by 1e3 eps). A fitted sum carries
+    the rounding of some 40 operations on terms of up to 3 (N) and 6 / h (grad N)."""
+    dtype = np.float32
+    from helpers import basis_kind
+    from tesserae_b200 import runtime
+    abi = tb._abi
+    h, x0 = 1.0 / 13, 100.3
+    cells = (11, 9, 10)[:dim]
+    mesh = tb.CartesianMesh(h, *[(x0, x0 + c * h) for c in cells])
+    rng = np.random.default_rng(17)
+    n = 4000
+    P = tb.Particles(n, dim, np.float64)
+    for d in range(dim):
+        P.x[d] = x0 + rng.uniform(0.02, cells[d] - 0.02, size=n) * h
+    P.x[0] = x0 + rng.uniform(0.02, 0.45, size=n) * h  # windows that the mesh cuts on one axis at least
+    Pd = P.to("torch", device="cuda", dtype=dtype)
+    W = tb.BasisWeights(dim, n, dtype, backend="torch", device="cuda")
+    prm = tb.step_params(1e-4, gimp_l=0.45 * h, basis=basis_kind(abi, basis))
+    runtime.update(W, Pd, mesh, prm, ctx=ctx)
+    ctx.synchronize()
+    w = W.w.cpu().numpy().astype(np.float64).reshape(n, -1)
+    g = W.grad_w.cpu().numpy().astype(np.float64).reshape(n, w.shape[1], dim)
+    eps = float(np.finfo(dtype).eps)
+    assert np.abs(w.sum(axis=1) - 1.0).max() <= 40 * 3 * eps
+    assert np.abs(g.sum(axis=1)).max() <= 40 * 6 / h * eps
