@@ -36,10 +36,16 @@ def _row_ptrs(a, k: int) -> list[int | None]:
     if a is None:
         return [None] * k
     if isinstance(a, np.ndarray):
-        base, step = a.ctypes.data, a.strides[0]
+        rows, base, step = a.shape[0] if a.ndim > 1 else 0, a.ctypes.data, a.strides[0]
+    elif type(a) in (list, tuple):  # rows that are tensors of their own
+        return [a[i].data_ptr() for i in range(k)]
     else:
-        base, step = a.data_ptr(), a.stride(0) * a.element_size()
-    return [base + i * step for i in range(k)]
+        rows, base, step = a.shape[0], a.data_ptr(), a.stride()[0] * a.itemsize
+    if rows < k:  # the rest would be addresses past the array
+        raise IndexError(f"an array of {k} rows is needed, this one has {rows}")
+    if not (base and step):
+        return [base or None] * k
+    return list(range(base, base + k * step, step))
 
 
 # ---------------------------------------------------------------------------
