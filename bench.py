@@ -11,7 +11,9 @@ are measured beside it, with their accuracy.
 
   python bench.py [--gpus N] [--steps K] [--warmup W] [--impl b200|reference]
 
-Prints one JSON line (rank 0). N > 1 (torchrun): every rank runs its own
+Prints one JSON line (rank 0) of at most 1500 characters, so that a log's tail holds
+all of it, and every other measurement (configurations, kernels, adjoint legs) as one
+line of detail on stderr. N > 1 (torchrun): every rank runs its own
 replica of the workload (weak scaling, no data exchange); time = max over ranks.
 `--impl reference` times the reference's CPU algorithm (the OpenMP restatement
 in oracle/, FP64, all host cores) on the same workload.
@@ -32,6 +34,39 @@ import numpy as np
 
 ROOT = pathlib.Path(__file__).resolve().parent
 METRIC = "particle-steps/s, 1 B200: FP32 fused vs FP64 plain @<=1e-5 rel err; adj/fwd"
+
+
+# What the result line keeps of the full measurement (a tuple: those keys of the entry).
+LINE_KEYS = {
+    "metric": None, "value": None, "unit": None, "n_gpus": None, "steps": None, "warmup": None, "ms_per_step": None,
+    "higher_is_better": None, "scaling": None, "vs_baseline": None, "dtype": None, "data": None,
+    "config": ("workload", "n_particles", "scale", "parallelism", "l2"),
+    "accuracy": ("steps", "rel_err_x", "rel_err_v"),
+    "fp64_plain": ("value",), "adjoint_over_forward": ("value", "backward_over_forward"),
+    "roofline": ("bound", "kernel", "achieved", "peak", "unit", "frac", "peak_source"),
+    "cpu_baseline": ("value", "cores", "kind"),
+    "e2e": ("value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step", "mpm_steps_per_call"),
+    "gpu_launches": None, "clocks": ("sm_mhz", "sm_max_mhz", "reasons"),
+}
+LINE_MAX = 1500
+
+
+def result_line(out: dict) -> str:
+    """The JSON line of a run: LINE_KEYS of `out`, numbers to 7 digits."""
+    def short(v):
+        return float(f"{v:.7g}") if isinstance(v, float) else v
+
+    line = {}
+    for key, sub in LINE_KEYS.items():
+        v = out.get(key)
+        if sub is not None and v is not None:
+            v = {k: short(v[k]) for k in sub if k in v}
+        line[key] = short(v)
+    for spare in ("cpu_baseline", "adjoint_over_forward", "fp64_plain", "accuracy", "roofline"):
+        if len(json.dumps(line)) <= LINE_MAX:
+            break
+        del line[spare]  # (never at the sizes of a full run)
+    return json.dumps(line)
 
 
 def load_package():
@@ -1132,7 +1167,8 @@ def main():
         "gpu_launches": hd["launches"],
         "clocks": hd["clocks"],
     }
-    print(json.dumps(out), flush=True)
+    print("bench detail: " + json.dumps(out), file=sys.stderr, flush=True)
+    print(result_line(out), flush=True)
     if dist is not None:
         dist.destroy_process_group()
 
