@@ -661,11 +661,13 @@ struct PairAcc {
 // evaluates the x and y jets once for 9 nodes instead of 3, so the per-record
 // overhead (loads, jets, row factors) is paid 3 times per particle instead of
 // 9; the 25 pencils x 3 z-slots are 75 lanes of the 128-thread CTA.
-// FULL: blocks at the mesh boundary run the same way (bspline_start), their
-// partials summed in FP64. Otherwise every block whose halo tile leaves the mesh is
-// appended to `bnd` for a launch with full records: the second gather costs the
-// interior blocks 2.6% (cube3d, 16.8 M particles: 1.047 against 1.020 ms), a second
-// launch 2 us.
+// FULL (B-spline): blocks at the mesh boundary run the same way (bspline_start), their
+// partials summed in FP64. Otherwise (KernelCorrection, whose cut windows have other
+// weights) every block whose halo tile leaves the mesh is appended to `bnd` for a
+// launch with full records. Whole steps of the B-spline with one launch and with two:
+// 34 k particles on a floor 48 / 60 us, 1.0 M in mid-mesh 208 / 211, 1.3 M on a floor
+// 241 / 275, 16.8 M in mid-mesh 2355 / 2358, 17.6 M on a floor 2480 / 2559 (FP32 with
+// FP64 positions).
 constexpr int PLANE_THREADS = 128;
 constexpr int PLANE_NR = 512;
 constexpr int CRS = 14;  // words of a PairRec record
@@ -1336,8 +1338,6 @@ cudaError_t launch_p2g_2d(const DMesh<2, T>& M, const PView<T>& P, const GView<T
 }
 
 
-constexpr int PLANE_ONE_BLOCKS = 16384;  // a 100^3-cell mesh
-
 // 3D. The quadratic B-spline in the FP32 forms takes the plane kernel (short
 // records, 9 nodes per lane). KernelCorrection changes the weights of cut windows
 // only: its interior blocks are plain B-spline, the others (their list in binning
@@ -1353,12 +1353,8 @@ cudaError_t launch_p2g_3d(const DMesh<3, T>& M, const PView<T>& P, const GView<T
                    : launch_pencil<T, X64, P_APIC>(M, P, G, s, b, cfg);
     if (wls) return launch_pencil<T, X64, P_WLS>(M, P, G, s, b, cfg);
     if constexpr (sizeof(T) == 4) {
-        // one launch where it is worth its 2 us: P2G takes 2.6% less with two, which
-        // is 2 us from about 1 M particles on; up to PLANE_ONE_BLOCKS mesh blocks a
-        // B-spline takes one
-        if (s.basis == TB_BSPLINE_QUADRATIC && M.nblocks <= PLANE_ONE_BLOCKS)
-            return launch_plane<X64, true>(M, P, G, s, b, cfg, nullptr, nullptr);
-        if (s.basis == TB_BSPLINE_QUADRATIC || s.basis == TB_KC_BSPLINE_QUADRATIC) {
+        if (s.basis == TB_BSPLINE_QUADRATIC) return launch_plane<X64, true>(M, P, G, s, b, cfg, nullptr, nullptr);
+        if (s.basis == TB_KC_BSPLINE_QUADRATIC) {
             const cudaError_t e = launch_plane<X64, false>(M, P, G, s, b, cfg, b.cursors, b.bnd_count);
             if (e != cudaSuccess) return e;
             return launch_pencil<T, X64, P_JET>(M, P, G, s, b, cfg, b.cursors, b.bnd_count);
