@@ -510,6 +510,7 @@ int run_step(tb_ctx* c, const tb_mesh* m, tb_particles* p, tb_partition* part, t
     if ((rc = make_gview<T>(c, g, D, G, m->block_log2)) != TB_OK) return rc;
     BinBuffers B;
     if ((rc = bin_buffers(c, part, P.n, M.nblocks, B)) != TB_OK) return rc;
+    B.fresh = do_bin;
     const LaunchCfg cfg = cfg_of(c, P.n);
     const T* xs[3] = {P.x[0], P.x[1], D == 3 ? P.x[2] : P.x[1]};
     // FP64 positions are binned by the FP64 findblock (the reference's Float64 rule)
@@ -945,6 +946,7 @@ int g2p2g_impl(tb_ctx* c, const tb_mesh* m, tb_particles* p, tb_partition* part,
     if (G.bnum) return fail(c, TB_ERR_UNSUPPORTED, "g2p2g runs on a dense grid");
     BinBuffers B;
     if ((rc = bin_buffers(c, part, P.n, M.nblocks, B)) != TB_OK) return rc;
+    B.fresh = true;  // binned below; P2G reads the positions before the move
     if ((rc = touched_buffers(c, M.nblocks)) != TB_OK) return rc;
     const size_t xe = x64 ? sizeof(double) : sizeof(T);
     cudaError_t e = grow(c->g2p2g_x, c->g2p2g_x_cap,

@@ -19,6 +19,7 @@ struct BinBuffers {
     unsigned long long* sort_scratch;  // [2n] scratch for large blocks
     int* totals;          // [2] device: nactive, nassigned
     unsigned long long* bnd_count;  // [1] blocks P2G leaves to its second launch; zeroed by every binning
+    bool fresh = false;   // the partition is that of the positions P2G reads
 };
 
 // Node blocks that a step's transfer touches, found by the scan of its binning:

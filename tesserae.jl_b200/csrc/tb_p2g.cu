@@ -79,7 +79,6 @@ __device__ __forceinline__ bool window_start(const DMesh<D, T>& M, const Scalars
 
 // Whether a position lies in the mesh (findblock's rule). Every particle of a fresh
 // partition does; one that has left the mesh since the binning has no support there.
-// The check costs the FP64 B-spline step of 917 k particles 2.5 us of 341.
 template <int D, class T, bool X64>
 __device__ __forceinline__ bool inside_mesh(const DMesh<D, T>& M, const double* xd, const T* x) {
     bool in = true;
@@ -297,10 +296,11 @@ struct Fields {
         }
     }
     // Window start per axis (unclipped for P_BSP, whose t it also leaves in x);
-    // false for a particle that takes no part (P_BSP: outside the mesh).
+    // false for a particle that takes no part (P_BSP, with STALE: outside the mesh).
+    template <bool STALE>
     __device__ __forceinline__ bool window(const DMesh<3, T>& M, const Scalars<T>& s, int (&lo)[3], int* err) {
         if constexpr (KIND == P_BSP) {
-            const bool in = inside_mesh<D, T, X64>(M, xd, x);
+            const bool in = !STALE || inside_mesh<D, T, X64>(M, xd, x);
 #pragma unroll
             for (int d = 0; d < D; ++d) {
                 T t;
@@ -384,7 +384,9 @@ struct Fields {
 // 0.196 ms with full records, 0.177 ms with compact ones.
 constexpr int P2G_THREADS = 288;
 
-template <class T, bool X64, int KIND, int NR, int CTAS>
+// STALE (P_BSP): the partition may be older than the positions. A fresh one holds no
+// particle outside the mesh, and the check costs a step of 125 k particles 2.5 us of 89.
+template <class T, bool X64, int KIND, int NR, int CTAS, bool STALE>
 __global__ void __launch_bounds__(P2G_THREADS, CTAS)
     p2g_pencil_kernel(DMesh<3, T> M, PView<T> P, GView<T> G, Scalars<T> s, const int* __restrict__ totals,
                       const int* __restrict__ blocklist, const int* __restrict__ offsets,
@@ -460,7 +462,7 @@ __global__ void __launch_bounds__(P2G_THREADS, CTAS)
                 rank[u] = 0;
                 int lo[3];
                 if (pid[u] < 0) continue;
-                const bool in = f[u].window(M, s, lo, err);
+                const bool in = f[u].template window<STALE>(M, s, lo, err);
                 if (KIND != P_BSP && !in) continue;
                 int gi = 0;
                 bool ok = true;
@@ -470,7 +472,7 @@ __global__ void __launch_bounds__(P2G_THREADS, CTAS)
                     ok = ok && q >= 0 && q < G1;
                     gi = gi * G1 + q;
                 }
-                if (!ok || !in) {  // P_BSP: one branch for both (a branch each: P2G 2% slower)
+                if (!ok || !in) {
                     if (in) atomicOr(err, ERR_TILE_RANGE);
                     continue;
                 }
@@ -620,7 +622,9 @@ cudaError_t launch_pencil(const DMesh<3, T>& M, const PView<T>& P, const GView<T
                           const BinBuffers& b, const LaunchCfg& cfg, const int* list = nullptr,
                           const unsigned long long* nlist = nullptr) {
     constexpr int NR = pencil_nr<T, KIND>();
-    auto kern = p2g_pencil_kernel<T, X64, KIND, NR, sizeof(T) == 4 ? 2 : 1>;
+    constexpr int CTAS = sizeof(T) == 4 ? 2 : 1;
+    auto kern = p2g_pencil_kernel<T, X64, KIND, NR, CTAS, KIND == P_BSP>;
+    if (KIND == P_BSP && b.fresh) kern = p2g_pencil_kernel<T, X64, KIND, NR, CTAS, false>;
     const size_t smem = pencil_smem_bytes<T, KIND, NR>();
     int grid = 0;
     cudaError_t e = prepare_launch(kern, P2G_THREADS, smem, cfg, M.nblocks, grid);
