@@ -65,11 +65,13 @@ struct LaunchCfg {
 };
 
 // Scenes up to this many particles set their blocks up early: a launch is then a
-// good part of its kernel. Above it the kernels fill the GPU, and blocks that arrive
-// while the launch before still runs disturb it (1.9 M-particle sphere, 8 steps: 4.89 ms
-// in order, 5.06 early; 917 k-particle FP64 block, one step: 362 us in order, 345 early;
-// 111 k-particle 2D scene, 25 steps: 1.74 ms in order, 1.46 early).
-constexpr long long EARLY_N = 1 << 20;
+// good part of its kernel. Whole steps early / in order, us: 2D 361 k particles 79.5 / 91.6;
+// 3D FP32 with FP64 positions 262 k 76 / 88, 1.0 M 190 / 202, 2.7 M 473 / 479, 8.0 M 1195 / 1199,
+// 16.8 M 2338 / 2324; FP64 512 k 175 / 179, 2.7 M 788 / 794, 5.8 M 1518 / 1516; WLS + APIC 2.6 M 743 / 759,
+// 18 M 5069 / 5065. Two kernels follow in order where they lose by it (p2g_plane_kernel;
+// bin_fixup_kernel in crowded scenes): their large blocks arrive on SMs that still run the
+// launch before.
+constexpr long long EARLY_N = 1 << 23;
 
 // Launches of a step follow each other on one stream; each waits for the one before
 // on the device (chain_wait, its first statement) instead of at launch, so that its

@@ -981,7 +981,12 @@ cudaError_t launch_plane(const DMesh<3, float>& M, const PView<float>& P, const 
     int grid = 0;
     cudaError_t e = prepare_launch(kern, PLANE_THREADS, smem, cfg, M.nblocks, grid);
     if (e != cudaSuccess) return e;
-    launch_chained(kern, grid, PLANE_THREADS, smem, cfg, M, P, G, s, b.totals, b.blocklist, b.offsets, b.perm, cfg.err,
+    // In order: set up early, its blocks (76 KB of shared memory, three per SM) arrive where
+    // the fix-up still runs, and whole steps of 0.5 M particles and more take 2 to 10%
+    // longer (1.0 M: 209 us early, 202 with every launch in order, 191 with this one).
+    LaunchCfg in_order = cfg;
+    in_order.early = false;
+    launch_chained(kern, grid, PLANE_THREADS, smem, in_order, M, P, G, s, b.totals, b.blocklist, b.offsets, b.perm, cfg.err,
                                                    bnd, bnd_count);
     ++*cfg.launches;
     return cudaGetLastError();
