@@ -84,3 +84,40 @@ def test_wls_weights_reproduce_constants_far_from_the_origin(tb, ctx, dim, basis
     eps = float(np.finfo(dtype).eps)
     assert np.abs(w.sum(axis=1) - 1.0).max() <= 40 * 3 * eps
     assert np.abs(g.sum(axis=1)).max() <= 40 * 6 / h * eps
+
+
+def test_ugimp_quotient_is_the_division_to_one_ulp(tb, ctx):
+    """The uGIMP jets divide by the particle's length through its inverse, corrected once.
+    At FP32, with offsets that are exact (h = 1/8, positions of few bits) and a second
+    axis whose weight is 1/2, grad N gives the jet's derivative itself: 2 a / l or
+    (1 + l/2 - a) / l, at most one ulp from the division."""
+    from tesserae_b200 import runtime
+    abi = tb._abi
+    f = np.float32
+    h, cells, n = 0.125, 16, 20000
+    mesh = tb.CartesianMesh(h, (0.0, cells * h), (0.0, cells * h))
+    rng = np.random.default_rng(23)
+    P = tb.Particles(n, 2, np.float32, optional=("l",))
+    P.x[0] = (rng.integers(4 * 4096, 12 * 4096, size=n) / 4096).astype(f) * f(h)
+    P.x[1] = f(8.5 * h)
+    P.l[...] = rng.uniform(0.05, 0.95, size=n).astype(f) * f(h)
+    Pd = P.to("torch", device="cuda", dtype=np.float32)
+    W = tb.BasisWeights(2, n, np.float32, backend="torch", device="cuda")
+    runtime.update(W, Pd, mesh, tb.step_params(1e-4, gimp_l=0.5 * h, basis=abi.TB_UGIMP), ctx=ctx)
+    ctx.synchronize()
+    gx = W.grad_w.cpu().numpy().reshape(n, 3, 3, 2)[..., 0]  # slots: x fastest
+    lo = W.window.cpu().numpy()
+    xi, l = P.x[0] * f(8), P.l * f(8)
+    r = f(1) + l / f(2)
+    first = np.floor(xi - r) + f(1)
+    checked = 0
+    for k in range(3):
+        a = np.abs(xi - (first + f(k)))
+        hl = l * f(0.5)
+        ref = np.where(a < hl, (f(2) * a) / l, np.where(a < f(1) - hl, f(1),
+                       np.where(a < f(1) + hl, (f(1) + hl - a) / l, f(0)))).astype(f)
+        der = np.abs(gx[:, 0, k]) * f(2) * f(h)  # the first y slot has weight 1/2
+        on = (first + f(k)) <= np.floor(xi + r)
+        assert np.all(np.abs(der - ref)[on] <= np.spacing(ref)[on]), k
+        checked += int(on.sum())
+    assert checked > 2 * n and lo.shape[0] == n

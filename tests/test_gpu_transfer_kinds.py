@@ -67,13 +67,74 @@ def test_one_step(tb, oracle, ctx, dim, ppc, sparse, basis, transfer, form):
         scale = max(np.abs(ref).max(), {"m": 1.3, "mv": 1.3, "f": 1.0 / mesh.h}[k])
         assert np.abs(g[k] - ref).max() <= tol * scale, k
     got = Pd.numpy()
+    # two cells from every face no window is cut by the mesh
+    inner = np.all([(P.x[d] > 2 * mesh.h) & (P.x[d] < (mesh.n_nodes[d] - 3) * mesh.h) for d in range(dim)], axis=0)
     for k in ("v", "F") + (("B",) if transfer == "apic" else ()):
         ref = getattr(Po, k)
         scale = np.abs(ref).max()
-        # nodes that a single window barely touches divide two sums near zero: FP32
-        # weights there carry the rounding of the position relative to the support
-        frac = np.mean(np.abs(got[k] - ref) > (tol if form == "f64" else 10 * tol) * scale)
-        assert frac <= (0.0 if form == "f64" else 2e-3), (k, frac)
+        assert np.isfinite(got[k]).all(), k
+        err = np.abs(got[k] - ref) / scale
+        if form == "f64":
+            assert (err <= tol).all(), (k, err.max())
+            continue
+        # FP32 positions carry eps |x| / h, 8e-7 of a cell. Inside, some ten such terms of
+        # 1 to 1 / h add up; a WLS fit beside a face divides by the variance of a cut window
+        # (down to 1/15 of h^2 per axis at 0.02 h from the face), 3e-3 in a corner: a few
+        # particles may be off by more than inside, none by more than that allows.
+        assert (err[:, inner] <= 10 * tol).all(), (k, err[:, inner].max())
+        assert np.mean(err > 10 * tol) <= 2e-3, k
+        assert (err <= 1e-2).all(), (k, err.max())
+
+
+@pytest.mark.parametrize("form", ["f64", "f32", "f32x64"])
+@pytest.mark.parametrize("transfer", ["flip", "apic"])
+@pytest.mark.parametrize("basis", BASES)
+@pytest.mark.parametrize("dim,ppc,sparse", [(3, 7, False), (3, 1, True), (2, 12, False), (2, 1, True)])
+def test_steps_of_one_call(tb, oracle, ctx, dim, ppc, sparse, basis, transfer, form):
+    """Four fused steps in one call, which zero and update the touched blocks only, count
+    the particles of the next step in G2P and (these scenes are small) set launches up
+    early, against the oracle's; the grid is that of the last step on every node. The
+    particles move a third of a cell, so blocks are entered and left."""
+    from helpers import basis_kind, rel_l2
+    from tesserae_b200 import runtime
+    if form == "f32x64" and dim == 2 and (transfer == "apic" or basis.startswith("wls")):
+        pytest.skip("refused: the FP64-position form runs WLS and APIC in 3D only")
+    abi = tb._abi
+    mesh, P = _scene(tb, dim, ppc, sparse, 11 * dim + ppc)
+    h = mesh.h
+    rng = np.random.default_rng(5)
+    hi = np.array([(n - 1) * h for n in mesh.n_nodes])[:, None]
+    P.x[...] = np.clip(P.x, 2.0 * h, hi - 2.0 * h)  # whole windows throughout
+    P.x[...] += 0.01 * h * rng.uniform(-1.0, 1.0, size=P.x.shape)
+    P.v[...] = 0.05 * P.v + np.array([0.8, -0.6, 0.7])[:dim, None]
+    P.sigma[...] *= 1e-3
+    dtype = np.float64 if form == "f64" else np.float32
+    dt = 0.1 * h
+    prm = tb.step_params(dt, mass=1.3, V0=1.0, mu=1e-3, lam=1e-3, gravity=(0.1, -0.2, 0.3)[:dim], gimp_l=0.45 * h,
+                         flip_alpha=0.9, basis=basis_kind(abi, basis),
+                         transfer=abi.TB_TRANSFER_APIC if transfer == "apic" else abi.TB_TRANSFER_FLIP)
+    Pd = P.to("torch", device="cuda", dtype=dtype, x64=form == "f32x64")
+    Po = Pd.to("numpy", dtype=np.float64, x64=False)
+    part = tb.Partition(mesh, P.n, backend="torch", device="cuda")
+    G = tb.generate_grid(mesh, dtype, backend="torch", device="cuda")
+    for k in ("m", "mv", "f", "v", "vn"):
+        getattr(G, k).fill_(3.0)  # what an earlier run left
+    runtime.step(G, Pd, part, mesh, prm, 4, ctx=ctx)
+    ctx.synchronize()
+    Go = tb.generate_grid(mesh, np.float64)
+    oracle.step(mesh, Po, Go, prm, 4)
+    got, g = Pd.numpy(), G.numpy()
+    tol = 1e-10 if form == "f64" else 1e-3
+    for k in ("x", "v", "F") + (("B",) if transfer == "apic" else ()):
+        assert np.isfinite(got[k]).all(), k
+        assert rel_l2(got[k], getattr(Po, k)) <= tol, (k, rel_l2(got[k], getattr(Po, k)))
+    for k in ("m", "mv"):
+        assert np.isfinite(g[k]).all(), k
+        ref = getattr(Go, k)
+        assert rel_l2(g[k].reshape(ref.shape), ref) <= tol, (k, rel_l2(g[k].reshape(ref.shape), ref))
+    bare = Go.m == 0.0
+    for k in ("v", "vn"):  # nodes that no particle of the last step reaches read as zero
+        assert np.all(g[k].reshape((dim,) + Go.m.shape)[:, bare] == 0.0), k
 
 
 @pytest.mark.parametrize("stretch", [1e-4, 0.02, 0.06, 0.2])
