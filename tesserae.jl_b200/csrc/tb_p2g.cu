@@ -371,8 +371,8 @@ struct Fields {
 // the 25 pencils. After each group the x-node the window leaves for good is final
 // for this (pencil, row) and is stored to the lane's own slot of the staging
 // array. A block's later batches add to the staged sums, so the gather and the
-// global atomics run once per block and piece. The partials are summed in FP32 on
-// interior blocks of the general FP32 kinds (WLS, APIC), in FP64 else.
+// global atomics run once per block and piece. The staged partials of a node are
+// summed in T for the general kinds (WLS, APIC), in FP64 for the others.
 // What bounds it is the chain of a batch (load, rank, record, sweep of the longest
 // pencil of a warp) at two CTAs of 9 warps per SM in FP32 and one in FP64, whose
 // staging array takes 88 KB: issue slots are about a third used, so the general
@@ -380,7 +380,7 @@ struct Fields {
 // shared, but each record's chain is twice as long and a third of the warps run).
 // Dam break at half resolution (18.2 M particles, WLS(uGIMP) + APIC, FP32 with FP64
 // positions): 6.03 ms with a moment inverse at every node of a plane lane, 4.04 ms
-// with the closed form on plane lanes, 3.06 ms here. FP64 B-spline, 917 k particles:
+// with the closed form on plane lanes, 2.98 ms here. FP64 B-spline, 917 k particles:
 // 0.196 ms with full records, 0.177 ms with compact ones.
 constexpr int P2G_THREADS = 288;
 
@@ -430,14 +430,12 @@ __global__ void __launch_bounds__(P2G_THREADS, CTAS)
         const int li = split == 1 ? vi : vi / split, piece = vi - li * split;
         const int b = list ? list[li] : blocklist[li] - 1;
         int org[3];
-        bool interior = true;
         {
             int r = b;
 #pragma unroll
             for (int d = 0; d < 3; ++d) {
                 org[d] = (r % M.nb[d]) * 4 - 1;
                 r /= M.nb[d];
-                interior = interior && org[d] >= 0 && org[d] + TS - 1 <= M.n[d] - 1;
             }
         }
         const int s0 = offsets[b], s1 = offsets[b + 1];
@@ -1003,14 +1001,14 @@ cudaError_t launch_plane(const DMesh<3, float>& M, const PView<float>& P, const 
 // 2D scenes are small: what bounds this kernel is the chain of a piece (load, rank,
 // record, three classes, gather). 25 steps of a 111 k particle WLS + APIC scene in FP32: 0.185
 // ms per step with one lane per pencil row, a moment inverse at every node and FP64
-// shared atomics; 0.040 ms here.
+// shared atomics; 0.027 ms here.
 //
 // Record (words of T, in pairs): 0 (m, m v_x)  2 (m v_y, S11)  4 (S00, S01)
 //   Q_BSP   quadratic B-spline, FLIP: 6 (t_x, t_y)
 //   others  6 + 2j (wy, gy), 12 + 2i (wx, gx): jets (value, gradient)
 //   Q_WLS   18 (u_x, u_y)
 //   Q_APIC  (plain kernel) 18, Q_WLS_APIC 20: (B00, B10) (B01, B11) (r0_x, r0_y), B = m D^-1 B_p
-// S = -V sigma; the weights and sums are those of the general plane kernel.
+// S = -V sigma; the weights and sums are those of the pencil kernel, without z.
 enum : int { Q_BSP = 0, Q_JET = 1, Q_WLS = 2, Q_WLS_APIC = 3, Q_APIC = 4 };
 
 template <int KIND>
@@ -1345,7 +1343,6 @@ cudaError_t launch_p2g_2d(const DMesh<2, T>& M, const PView<T>& P, const GView<T
     if (s.basis == TB_BSPLINE_QUADRATIC) return launch_2d_kind<T, BW, X64, Q_BSP>(M, P, G, s, b, cfg);
     return launch_2d_kind<T, BW, X64, Q_JET>(M, P, G, s, b, cfg);
 }
-
 
 // 3D. The quadratic B-spline in the FP32 forms takes the plane kernel (short
 // records, 9 nodes per lane). KernelCorrection changes the weights of cut windows
