@@ -1,5 +1,5 @@
 """The general device reverse step (WLS and KernelCorrection bases, APIC; the
-particle-parallel kernels with Dual3 weight derivatives) through the C ABI
+particle-parallel kernels with Dual1 weight derivatives) through the C ABI
 against the oracle's general reverse step, which tests/test_adjoint_general.py
 pins to forward-mode dual numbers: one step (FP64 to 1e-10 relative L2 per
 field, the mixed FP32 form to 1e-4) and the checkpointed tape over several
