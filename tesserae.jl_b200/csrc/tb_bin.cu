@@ -526,11 +526,13 @@ __global__ void __launch_bounds__(FIX_THREADS) bin_fixup_kernel(const int* __res
 
 inline unsigned grid_for(long long n, int threads) { return unsigned((n + threads - 1) / threads); }
 
-// The fix-up is set up early up to this many particles per mesh block. Whole steps
-// with it early / in order, us: spheres in lattice order of 352 per mesh block (463 k)
-// 197 / 180, of 386 (1.9 M) 582 / 581, of 147 (195 k) 117 / 111; a block of 57 (512 k) 116.8 / 117.4,
-// a column in block order of 135 (454 k) 117.3 / 118.4, a sphere in block order of 147 132.5 / 133.3.
-constexpr long long FIX_EARLY_PER_BLOCK = 128;
+// The fix-up is set up early up to this many particles, in all and per mesh block.
+// Whole steps with it early / in order, us: spheres in lattice order of 352 per mesh
+// block (463 k) 197 / 180, of 386 (1.9 M) 582 / 581, of 147 (195 k) 117 / 111; a block of 57
+// (512 k) 116.8 / 117.4, a column in block order of 135 (454 k) 117.3 / 118.4, a sphere in block
+// order of 147 132.5 / 133.3. Blocks of 58 in lattice order: 1.7 M 498 / 500, 2.7 M 913 / 899,
+// 3.5 M 1033 / 1022, 4.9 M 1489 / 1491; in block order 2.7 M 622 / 616.
+constexpr long long FIX_EARLY_N = 1 << 21, FIX_EARLY_PER_BLOCK = 128;
 
 constexpr int SCAN_ONE = 16;  // tiles up to which the scan is one launch
 
@@ -629,7 +631,7 @@ cudaError_t launch_bin_rest(int nb, long long n, const BinBuffers& b, const Laun
         KernelScope ks(cfg, "bin_fixup");
         const int grid = std::max(1, std::min(nb, cfg.num_sms * 5));
         LaunchCfg fix = cfg;
-        fix.early = cfg.early && n <= FIX_EARLY_PER_BLOCK * nb;
+        fix.early = cfg.early && n <= FIX_EARLY_N && n <= FIX_EARLY_PER_BLOCK * nb;
         launch_chained(bin_fixup_kernel, grid, FIX_THREADS, 0, fix, b.totals, b.blocklist, b.offsets, b.perm_tmp, b.perm,
                                                                b.sort_scratch, zero_counts ? b.counts : nullptr, nb);
         *cfg.launches += 2;
